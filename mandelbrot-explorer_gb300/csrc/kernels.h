@@ -184,6 +184,7 @@ struct ShallowParams {
     FrameGeom g;
     double c0r, c0i, dx, dy;
     int simd_semantics;      // 1: lane-refill kernel (float result), 0: floatPointCompute
+    unsigned esc_word = 0;   // direct_escape_word(g.ESC2), set by launch_shallow
 };
 
 // Julia frames (Mandel::ComputeJulia, mp.cpp:992-1044): z0 = c0 + (dx j, dy i).
@@ -191,6 +192,7 @@ struct JuliaParams {
     FrameGeom g;
     double z0r, z0i, dx, dy; // lower-left sample and spacings (mpf_get_ld)
     double cr, ci;           // the fixed c
+    unsigned esc_word = 0;   // direct_escape_word(g.ESC2), set by launch_julia
 };
 
 struct DeviceFrame {

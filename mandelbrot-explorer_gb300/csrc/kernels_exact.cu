@@ -7,6 +7,7 @@
 //
 // Reference: cbotx/Mandelbrot-Explorer src/engine/mandel_perturbation.cpp
 // ("mp.cpp"); the per-pixel semantics are those of its scalar loops.
+#include "direct_loop.cuh"
 #include "kernels.h"
 #include "orbit_color.h"
 
@@ -938,13 +939,14 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
 
 // ---------------------------------------------------------------------------
 // Shallow direct loop: floatPointCompute (mp.cpp:330-399) and the lane-refill
-// kernel's per-lane arithmetic (mp.cpp:416-532).
+// kernel's per-lane arithmetic (mp.cpp:416-532). The plain loops below, with the
+// interior test's derivative in FP64, take only the samples that
+// direct_iterate (direct_loop.cuh) leaves open.
 template <int OC>
-__device__ double shallow_scalar(double c_re, double c_im, int mxit, const FrameGeom& g, double* nrm, int* nout) {
+__device__ __noinline__ int shallow_scalar_plain(double c_re, double c_im, int mxit, const FrameGeom& g, DirectState& s, OrbitColor<OC>& oc) {
     double z_re = c_re, z_im = c_im, d_re = 2, d_im = 0, dc_re = 1, dc_im = 0, tmp;
     const bool deriv = g.ede || g.deovl || g.normal;
-    OrbitColor<OC> oc; // mp.cpp:347-369
-    oc.init();
+    oc.init(); // mp.cpp:347-369
     int i = 1;
     while (i < mxit) {
         tmp = 2.0 * (d_re * z_re - d_im * z_im);
@@ -961,29 +963,19 @@ __device__ double shallow_scalar(double c_re, double c_im, int mxit, const Frame
         oc.push(z_re, z_im);
         tmp = z_re * z_re + z_im * z_im;
         if (tmp > g.ESC2) {
-            *nout = i + 1;
-            if (g.ede) return sqrt(tmp) * log(tmp) / sqrt(dc_re * dc_re + dc_im * dc_im);
-            if (g.normal) { // mp.cpp:375-378
-                if (nrm) *nrm = atan2(z_im, z_re) - atan2(dc_im, dc_re);
-                return (i + 1 - log(log(tmp) / 2 / kLn2) / kLn2);
-            }
-            if (g.deovl) {
-                if (nrm) *nrm = sqrt(tmp) * log(tmp) / sqrt(dc_re * dc_re + dc_im * dc_im);
-                return (i + 1 - log(log(tmp) / 2 / kLn2) / kLn2);
-            }
-            if (OC) return oc.escaped(i + 1 - log(log(tmp) / 2 / kLn2) / kLn2, tmp, g.ER); // mp.cpp:383-389
-            return (i + 1 - log(log(tmp) / 2 / kLn2) / kLn2);
+            s = DirectState{z_re, z_im, tmp, dc_re, dc_im, i + 1};
+            return kDirectEscaped;
         }
         tmp = d_re * d_re + d_im * d_im;
-        if (tmp < 0.000000001) return oc.interior();
+        if (tmp < 0.000000001) return kDirectInterior;
         ++i;
     }
-    return oc.interior();
+    return kDirectInterior;
 }
 
-__device__ float shallow_lane(double cr, double ci, int mxit, const FrameGeom& g, int* nout) {
-    double zr = cr, zi = ci, dr = 2, di = 0, dcr = 1, dci = 0, jv = 1;
-    for (;;) {
+__device__ __noinline__ int shallow_lane_plain(double cr, double ci, int mxit, const FrameGeom& g, DirectState& s) {
+    double zr = cr, zi = ci, dr = 2, di = 0, dcr = 1, dci = 0;
+    for (int n = 1;; ++n) {
         double ndr = 2.0 * ((dr * zr) - (di * zi));
         double ndi = 2.0 * ((dr * zi) + (di * zr));
         double ndcr = (2.0 * ((dcr * zr) - (dci * zi))) + 1.0;
@@ -998,54 +990,100 @@ __device__ float shallow_lane(double cr, double ci, int mxit, const FrameGeom& g
         dci = ndci;
         double zrad = (zr * zr) + (zi * zi);
         double dmag = (dr * dr) + (di * di);
-        double jnext = jv + 1.0;
         if (zrad > g.ESC2) {
-            *nout = (int)jv + 1;
-            if (g.ede) return (float)(sqrt(zrad) * log(zrad) / sqrt(dcr * dcr + dci * dci));
-            return (float)(jv + 1 - log(log(zrad) / 2 / kLn2) / kLn2);
+            s = DirectState{zr, zi, zrad, dcr, dci, n + 1};
+            return kDirectEscaped;
         }
-        if (dmag < 1e-9) return -2.0f;
-        if (jnext >= (double)mxit) return -2.0f;
-        jv = jnext;
+        if (dmag < 1e-9 || n + 1 >= mxit) return kDirectInterior;
     }
 }
 
-// One Julia sample with the per-lane arithmetic of solveJuliaShallowSimdList
-// (mp.cpp:534-636): z0 the sample, c fixed, D_0 = 1 and D' = 2 z D under EDE.
-// nout: escape index (0 when z0 is already outside), -1 interior.
-__device__ float julia_lane(double zr, double zi, double cr, double ci, int mxit, const FrameGeom& g, int* nout) {
-    double zrad = (zr * zr) + (zi * zi);
-    *nout = -1;
-    if (zrad > g.ESC2) {
-        *nout = 0;
-        return g.ede ? (float)(sqrt(zrad) * log(zrad)) : (float)(-log(log(zrad) / 2 / kLn2) / kLn2);
-    }
-    double dr = 1.0, di = 0.0, jv = 0.0;
-    for (;;) {
-        double ndr = dr, ndi = di;
-        if (g.ede) {
-            ndr = 2.0 * ((dr * zr) - (di * zi));
-            ndi = 2.0 * ((dr * zi) + (di * zr));
-        }
-        const double nzr = ((zr * zr) - (zi * zi)) + cr;
-        const double nzi = (2.0 * (zr * zi)) + ci;
-        zr = nzr;
+// The distance sqrt(zrad) log(zrad) / |dz/dc|.
+__device__ __forceinline__ double direct_distance(const DirectState& s) {
+    return sqrt(s.zrad) * log(s.zrad) / sqrt(s.dcr * s.dcr + s.dci * s.dci);
+}
+// The lane kernel's value (float): the smooth count, or the distance under EDE; -2 interior.
+__device__ float shallow_lane(double cr, double ci, int mxit, const FrameGeom& g, unsigned esc_word, int* nout) {
+    DirectState s;
+    auto none = [](double, double, double, double) {};
+    int st = g.ede ? direct_iterate<true, true>(cr, ci, mxit, g.ESC2, esc_word, s, none) : direct_iterate<true, false>(cr, ci, mxit, g.ESC2, esc_word, s, none);
+    if (st == kDirectOpen) st = shallow_lane_plain(cr, ci, mxit, g, s);
+    if (st == kDirectInterior) return -2.0f;
+    *nout = s.n;
+    if (g.ede) return (float)direct_distance(s);
+    return (float)smooth_value(s.n, s.zrad);
+}
+
+// The stripe average of an escaped sample: its last kStripeWindow terms, from
+// the orbit iterated once more (the trigonometry of the other iterations, and
+// of every interior sample, is never formed; with at most a window of
+// iterations the sums are those of the reference operation for operation).
+__device__ __noinline__ float shallow_stripe(double cr, double ci, const DirectState& s, double ER) {
+    StripeTail tail;
+    tail.init();
+    double zr = cr, zi = ci, x2 = zr * zr, y2 = zi * zi;
+    const int first = s.n - kStripeWindow;
+    for (int k = 1; k < s.n; ++k) {
+        const double nzi = twice(zr) * zi + ci;
+        zr = (x2 - y2) + cr;
         zi = nzi;
-        dr = ndr;
-        di = ndi;
-        zrad = (zr * zr) + (zi * zi);
-        const double jnext = jv + 1.0;
-        if (zrad > g.ESC2) {
-            *nout = (int)jv + 1;
-            if (g.ede) {
-                const double denom = sqrt((dr * dr) + (di * di));
-                return denom > 0.0 ? (float)(sqrt(zrad) * log(zrad) / denom) : 0.0f;
-            }
-            return (float)(jv + 1 - log(log(zrad) / 2 / kLn2) / kLn2);
-        }
-        if (jnext >= (double)mxit) return -2.0f;
-        jv = jnext;
+        x2 = zr * zr;
+        y2 = zi * zi;
+        if (k >= first) tail.push(zr, zi);
     }
+    return tail.value(s.zrad, ER);
+}
+
+// floatPointCompute's value, its normal angle or overlay distance in *nrm.
+template <int OC>
+__device__ double shallow_scalar(double c_re, double c_im, int mxit, const FrameGeom& g, unsigned esc_word, double* nrm, int* nout) {
+    const bool deriv = g.ede || g.deovl || g.normal;
+    DirectState s;
+    int st;
+    DirectTrap trap;
+    if (OC & kOcTrap) {
+        trap.init();
+        auto visit = [&](double zr, double zi, double x2, double y2) { trap.push(zr, zi, x2, y2); };
+        st = deriv ? direct_iterate<false, true>(c_re, c_im, mxit, g.ESC2, esc_word, s, visit) : direct_iterate<false, false>(c_re, c_im, mxit, g.ESC2, esc_word, s, visit);
+    } else {
+        auto visit = [](double, double, double, double) {};
+        st = deriv ? direct_iterate<false, true>(c_re, c_im, mxit, g.ESC2, esc_word, s, visit) : direct_iterate<false, false>(c_re, c_im, mxit, g.ESC2, esc_word, s, visit);
+    }
+    OrbitColor<OC & kOcTrap> oc; // the trap; a stripe average is formed at the escape
+    if (st == kDirectOpen) st = shallow_scalar_plain<OC & kOcTrap>(c_re, c_im, mxit, g, s, oc);
+    else trap.give(oc);
+    if (st == kDirectInterior) return oc.interior();
+    *nout = s.n;
+    if (g.ede) return direct_distance(s);
+    const double mu = smooth_value(s.n, s.zrad);
+    if (g.normal) { // mp.cpp:375-378
+        if (nrm) *nrm = atan2(s.zi, s.zr) - atan2(s.dci, s.dcr);
+    } else if (g.deovl) {
+        if (nrm) *nrm = direct_distance(s);
+    } else if (OC & kOcTrap) { // mp.cpp:383-389
+        return oc.escaped(mu, s.zrad, g.ER);
+    } else if (OC & kOcStripe) {
+        return shallow_stripe(c_re, c_im, s, g.ER);
+    }
+    return mu;
+}
+
+// One Julia sample: z0 the sample, c fixed (julia_iterate). nout: escape index
+// (0 when z0 is already outside), -1 interior.
+__device__ float julia_lane(double zr, double zi, double cr, double ci, int mxit, const FrameGeom& g, unsigned esc_word, int* nout) {
+    DirectState s;
+    const int st = g.ede ? julia_iterate<true>(zr, zi, cr, ci, mxit, g.ESC2, esc_word, s) : julia_iterate<false>(zr, zi, cr, ci, mxit, g.ESC2, esc_word, s);
+    *nout = -1;
+    if (st == kDirectInterior) return -2.0f;
+    *nout = s.n;
+    if (g.ede) {
+        const double num = sqrt(s.zrad) * log(s.zrad);
+        if (s.n == 0) return (float)num;
+        const double denom = sqrt((s.dcr * s.dcr) + (s.dci * s.dci));
+        return denom > 0.0 ? (float)(num / denom) : 0.0f;
+    }
+    const double x = log(log(s.zrad) / 2 / kLn2) / kLn2;
+    return s.n == 0 ? (float)(-x) : (float)((double)s.n - x);
 }
 
 // ComputeJulia's frame (mp.cpp:1019-1041): every sample of the grid, the EDE
@@ -1062,7 +1100,7 @@ __global__ void __launch_bounds__(128) k_julia(DeviceFrame f, JuliaParams p) {
         const int i = s / g.W, j = s - i * g.W;
         const double imag = p.z0i + p.dy * i;
         int nout = -1;
-        float v = julia_lane(p.z0r + p.dx * j, imag, p.cr, p.ci, g.mxit, g, &nout);
+        float v = julia_lane(p.z0r + p.dx * j, imag, p.cr, p.ci, g.mxit, g, p.esc_word, &nout);
         if (g.ede && v >= 0.0f) v /= (float)p.dx;
         f.out.iter[s] = v;
         if (f.out.escN) f.out.escN[s] = nout;
@@ -1105,12 +1143,12 @@ __global__ void __launch_bounds__(128) k_shallow(DeviceFrame f, ShallowParams p)
         int nout = -1;
         double val;
         if (OC == 0 && p.simd_semantics) { // (no orbit colourings in the lane kernel, mp.cpp:1459)
-            val = (double)shallow_lane(cr, ci, g.mxit, g, &nout);
+            val = (double)shallow_lane(cr, ci, g.mxit, g, p.esc_word, &nout);
             if (g.ede && val >= 0) val /= p.dx;
             f.out.iter[idx] = (float)val;
         } else {
             double de = 0.0;
-            val = shallow_scalar<OC>(cr, ci, g.mxit, g, &de, &nout);
+            val = shallow_scalar<OC>(cr, ci, g.mxit, g, p.esc_word, &de, &nout);
             if (g.normal) { // mp.cpp:1504-1507 (with EDE also set: the raw distance, angle 0)
                 f.out.iter[idx] = (float)val;
                 if (f.out.normal) f.out.normal[idx] = (float)de;
@@ -1275,12 +1313,16 @@ cudaError_t launch_fe_pass(const DeviceFrame& f, const FeParams& p, int blocks, 
     }
     return cudaGetLastError();
 }
-cudaError_t launch_julia(const DeviceFrame& f, const JuliaParams& p, int blocks, int threads, cudaStream_t st) {
+cudaError_t launch_julia(const DeviceFrame& f, const JuliaParams& jp, int blocks, int threads, cudaStream_t st) {
+    JuliaParams p = jp;
+    p.esc_word = direct_escape_word(p.g.ESC2);
     k_julia<<<blocks, threads, 0, st>>>(f, p);
     return cudaGetLastError();
 }
 
-cudaError_t launch_shallow(const DeviceFrame& f, const ShallowParams& p, int blocks, int threads, cudaStream_t st) {
+cudaError_t launch_shallow(const DeviceFrame& f, const ShallowParams& sp, int blocks, int threads, cudaStream_t st) {
+    ShallowParams p = sp;
+    p.esc_word = direct_escape_word(p.g.ESC2);
     switch (p.g.oc) {
     case 0: k_shallow<0><<<blocks, threads, 0, st>>>(f, p); break;
     case kOcStripe: k_shallow<kOcStripe><<<blocks, threads, 0, st>>>(f, p); break;

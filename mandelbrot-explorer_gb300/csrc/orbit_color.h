@@ -72,6 +72,33 @@ struct StripeAvg {
     }
 };
 
+// The stripe average of a run of at most W terms: the same sums while no term
+// has left the window (every term still in it, `out` above always 0), without
+// the ring.
+struct StripeTail {
+    double run, tri, last;
+    int fill;
+
+    MBX_OC_HD void init() {
+        run = tri = last = 0.0;
+        fill = 0;
+    }
+    MBX_OC_HD void push(double zr, double zi) {
+        const double t = 0.5 + 0.5 * sin(7.0 * atan2(zi, zr));
+        last = t;
+        ++fill;
+        tri += (double)kStripeWindow * t - run;
+        run += t;
+    }
+    MBX_OC_HD float value(double zrad, double R) const {
+        StripeAvg a;
+        a.tri = tri;
+        a.last = last;
+        a.fill = fill;
+        return a.value(zrad, R);
+    }
+};
+
 struct OrbitTrap {
     double point2;  // min |z|^2
     double cross;   // min min(|Re z|, |Im z|)
@@ -118,6 +145,15 @@ struct OrbitColor {
         return sac.value(zrad, R);
     }
     MBX_OC_HD float interior() const { return (OC & kOcTrap) ? trap.value(0.0) : -2.0f; }
+};
+template <>
+struct OrbitColor<kOcTrap> { // the traps alone: no stripe window to carry
+    OrbitTrap trap;
+    MBX_OC_HD void init() { trap.init(); }
+    MBX_OC_HD void push(double zr, double zi) { trap.push(zr, zi); }
+    MBX_OC_HD void skipped() {}
+    MBX_OC_HD float escaped(double mu, double, double) const { return trap.value(mu); }
+    MBX_OC_HD float interior() const { return trap.value(0.0); }
 };
 template <>
 struct OrbitColor<0> { // no orbit colouring: nothing to carry
