@@ -1499,7 +1499,6 @@ FeParams Engine::fe_params(int mx_ref_it) const {
     p.int_rep = 1;
     p.interior_confirm = interior_confirm_;
     p.interior_eps2 = interior_eps2_;
-    p.fused = 1;
     // the reference's no-BLA lane kernel has no derivative and no orbit colourings (mp.cpp:2148)
     p.no_bla_kernel = (!use_bla_ && !deriv_ && !(cm_ & (8 | 32))) ? 1 : 0;
     p.ref_period_gt0 = ref_period_ > 0 ? 1 : 0;

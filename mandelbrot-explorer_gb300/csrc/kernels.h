@@ -172,7 +172,7 @@ struct FeParams {
     int mx_ref_it;
     int use_interior, int_rep, interior_confirm;
     double interior_eps2;
-    int fused;
+    unsigned esc_word = 0;   // direct_escape_word(g.ESC2), set by launch_fe_pass
     int no_bla_kernel;       // mp.cpp:2185-2193 solveRescaledSimd8NoBla semantics
     int ref_period_gt0;
     int cutoff_sensitive;

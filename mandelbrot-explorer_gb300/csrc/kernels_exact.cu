@@ -390,18 +390,23 @@ __device__ void fe_deriv_underflow(FE zr, FE zi, FE& SJ, double& jr, double& ji,
 }
 
 // tryBLAfe (mp.cpp:2883-2970).
-// wm2: wr * wr + wi * wi when the caller has it (else a negative value)
-__device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int s, FE& S, FE S2, double& wr, double& wi, double dr, double di, double ESC2, int mx_ref_it, double* ab,
-                          double wm2 = -1.0) {
+__device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int s, FE& S, FE S2, double& wr, double& wi, double dr, double di, double ESC2, int mx_ref_it, double* ab) {
     if (s < 1 || b.nlev == 0) return 0;
     int maxp = b.nlev - 1;
     int startp = (s == 1) ? maxp : __ffs(s - 1) - 1;
     if (startp > maxp) startp = maxp;
     if (startp < b.minlevel) return 0;
-    double w2 = wm2;
-    if (dbits(wm2) >> 63) w2 = wr * wr + wi * wi; // (not known)
-    FE dz2 = fe_mul(S2, fe_from(w2));
-    if (b.rmax2 <= 0.0 || !fe_abs_less(dz2, fe_from(b.rmax2))) return 0;
+    if (d_le_zero(b.rmax2)) return 0;
+    const FE rmax = fe_from(b.rmax2);
+    {
+        // |w|^2 >= (the larger part)^2 >= 2^(2 k), k its binade, so |dz|^2's
+        // exponent is at least S2.e + 2 k: above rmax2's, no radius holds
+        const unsigned h = umax_(hi_abs(wr), hi_abs(wi));
+        const int64_t lo = S2.e + 2 * ((int64_t)(h >> 20) - 1023);
+        if (h >= 0x20000000u && h < 0x5fe00000u && !d_is_zero(S2.m) && lo > rmax.e) return 0;
+    }
+    const FE dz2 = fe_mul(S2, fe_from(wr * wr + wi * wi));
+    if (!fe_abs_less(dz2, rmax)) return 0;
     for (int p = startp; p >= b.minlevel; --p) {
         int i = (s - 1) >> p;
         if (i >= b.size[p]) continue;
@@ -416,9 +421,14 @@ __device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int
         const double BIG = 1e150;
         double2 zl = Z[land];
         if (d_abs_less(nwr, BIG) && d_abs_less(nwi, BIG)) { // (finite, below 1e150)
-            double fr = zl.x + fe_to_double(fe_mul_d(S, nwr));
-            double fi = zl.y + fe_to_double(fe_mul_d(S, nwi));
-            if (d_abs_less(ESC2, fr * fr + fi * fi)) return 0; // > ESC2
+            // z = Z_land + S n: with each part of Z_land and of S n below 4, |z|^2
+            // is below 128, so only a bailout^2 below that needs z itself
+            const unsigned hn = umax_(hi_abs(nwr), hi_abs(nwi));
+            if (!(umax_(hi_abs(zl.x), hi_abs(zl.y)) < 0x40100000u && (int64_t)(hn >> 20) - 1022 + S.e <= 2 && d_abs_less(200.0, ESC2))) {
+                double fr = zl.x + fe_to_double(fe_mul_d(S, nwr));
+                double fi = zl.y + fe_to_double(fe_mul_d(S, nwi));
+                if (d_abs_less(ESC2, fr * fr + fi * fi)) return 0; // > ESC2
+            }
             double wm2 = nwr * nwr + nwi * nwi;
             if (d_is_zero(wm2)) {
                 if (periodic)
@@ -467,25 +477,26 @@ struct PixOut {
     int state; // 1 escaped, 2 interior, 4 cancelled
 };
 
-// The plain delta step of pixelRescaled: w' = (2 X + s w) w + d in the fused
-// form, 2 (X w) + s w^2 + d otherwise. On GB300 each FP64 instruction holds
-// its SM quarter's FP64 unit for 64 cycles, independent operands or not, so
-// the exact form's loops are bound by their count of FP64 instructions: the
-// doubling X + X (exact) is formed on the bit pattern, and the tests below
-// compare bit patterns (floatexp.h d_is_zero, d_abs_less, d_eq), with the
-// IEEE results.
-__device__ __forceinline__ void fe_plain_step(bool fused, double Xr, double Xi, double s, double wr, double wi, double dr, double di, double& nwr, double& nwi) {
-    if (fused) {
-        const double fR = d_twice(Xr) + s * wr;
-        const double fI = d_twice(Xi) + s * wi;
-        nwr = fR * wr - fI * wi + dr;
-        nwi = fR * wi + fI * wr + di;
-    } else {
-        double w2r = wr * wr - wi * wi, w2i = 2.0 * wr * wi;
-        nwr = 2.0 * (Xr * wr - Xi * wi) + s * w2r + dr;
-        nwi = 2.0 * (Xr * wi + Xi * wr) + s * w2i + di;
-    }
+// The plain delta step of pixelRescaled in the fused form, w' = (2 X + s w) w + d,
+// with the products sw = s w of the current state.
+// On GB300 each FP64 instruction holds its SM quarter's FP64 unit for 64
+// cycles, independent operands or not, so the exact form's loops are bound by
+// their count of FP64 instructions (compares included), while about thirty
+// integer ones fit beside each. A common step therefore forms only what the
+// next state needs: the doubling X + X (exact) on the bit pattern, the step,
+// s w' once (for z now and for the next step), and z: 14 FP64 instructions. The
+// tests of a step are made on high words, exact tests on the bit patterns
+// (floatexp.h d_is_zero, d_abs_less, d_eq) only where those leave them open.
+__device__ __forceinline__ void fe_plain_step(double Xr, double Xi, double swr, double swi, double wr, double wi, double dr, double di, double& nwr, double& nwi) {
+    const double fR = d_twice(Xr) + swr;
+    const double fI = d_twice(Xi) + swi;
+    nwr = fR * wr - fI * wi + dr;
+    nwi = fR * wi + fI * wr + di;
 }
+// High words of a part's magnitude that settle a step's tests without FP64:
+// from kFeNearWord (just above 1e-4) on, |z|^2 >= 1e-8; in [kFeWLo, kFeWHi)
+// (just above 1e-8, 7e7) the larger part of w keeps |w|^2 within [1e-16, 1e16].
+constexpr unsigned kFeNearWord = 0x3f1a36e3u, kFeWLo = 0x3e45798fu, kFeWHi = 0x4190b076u;
 // |x| < 2^-1056 (the subnormal 2^18 * 2^-1074): the step's underflow test, on
 // the bit pattern
 __device__ __forceinline__ bool below_step_floor(double x) { return (dbits(x) & 0x7fffffffffffffffull) < 0x40000ull; }
@@ -514,6 +525,7 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
     }
     double s = fe_to_double(S);
     FE S2 = fe_mul(S, S);
+    double swr = s * wr, swi = s * wi; // kept with s and w
     int m = 1, iter = 1;
     double zsr = 1e30, zsi = 1e30;
     int save_iter = 1, period_win = 1;
@@ -526,32 +538,27 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
     const bool int_rep = p.int_rep && detect && !(OC & kOcTrap);
     OrbitColor<OC> oc;
     oc.init();
-    double swr = 1e300, swi = 1e300;
+    double rwr = 1e300, rwi = 1e300;
     FE sS = fe_make(1e300, 0);
     int sm = -1, save_iter2 = 1, twin2r = 1;
     PixOut o;
     o.nrm = 0.0f;
     o.n = -1;
     int tick = 0;
-    // |w|^2 of the current state when the previous iteration formed it (a
-    // step with no rescale or rebase after it), else -1
-    double wm2_known = -1.0;
     while (iter < g.mxit) {
-        const double wm2_now = wm2_known;
-        wm2_known = -1.0;
         if (((++tick) & 4095) == 0 && cancelled(f)) {
             o.state = 4;
             return o;
         }
         if (int_rep) {
-            if (m == sm && d_eq(wr, swr) && d_eq(wi, swi) && d_eq(S.m, sS.m) && S.e == sS.e) {
+            if (m == sm && d_eq(wr, rwr) && d_eq(wi, rwi) && d_eq(S.m, sS.m) && S.e == sS.e) {
                 o.value = -2.0f;
                 o.state = 2;
                 return o;
             }
             if (iter - save_iter2 >= twin2r) {
-                swr = wr;
-                swi = wi;
+                rwr = wr;
+                rwi = wi;
                 sS = S;
                 sm = m;
                 save_iter2 = iter;
@@ -560,7 +567,7 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
         }
         if (f.bla.use && !(OC & kOcTrap) && m >= 2) {
             double ab[4];
-            int skip = bla_try_fe(f.bla, Z, p.ref_period_gt0, rm, S, S2, wr, wi, dr, di, g.ESC2, per ? per : reflen, deriv ? ab : nullptr, wm2_now);
+            int skip = bla_try_fe(f.bla, Z, p.ref_period_gt0, rm, S, S2, wr, wi, dr, di, g.ESC2, per ? per : reflen, deriv ? ab : nullptr);
             if (skip > 0) {
                 ++n_bla;
                 n_skip += skip;
@@ -588,6 +595,8 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
                 S2 = fe_mul(S, S);
                 dr = fe_to_double(fe_div(dcr, S));
                 di = fe_to_double(fe_div(dci, S));
+                swr = s * wr;
+                swi = s * wi;
                 zsr = 1e30;
                 zsi = 1e30;
                 save_iter = iter;
@@ -604,8 +613,8 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
         double zmr = 0.0, zmi = 0.0;
         bool deriv_underflow = false;
         if (deriv) {
-            zmr = Xr + s * wr;
-            zmi = Xi + s * wi;
+            zmr = Xr + swr;
+            zmi = Xi + swi;
             deriv_underflow = d_is_zero(zmr) && d_is_zero(zmi) && d_is_zero(invSJd);
         }
         FE zmrfe = fe_make(0, 0), zmife = fe_make(0, 0);
@@ -616,7 +625,7 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
             zmife = fe_add(Xife, fe_mul_d(S, wi));
         }
         double nwr, nwi;
-        fe_plain_step(p.fused, Xr, Xi, s, wr, wi, dr, di, nwr, nwi);
+        fe_plain_step(Xr, Xi, swr, swi, wr, wi, dr, di, nwr, nwi);
         const bool step_underflow = below_step_floor(nwr) && below_step_floor(nwi);
         if (step_underflow && !(d_is_zero(nwr) && d_is_zero(nwi) && d_is_zero(wr) && d_is_zero(wi) && d_is_zero(dcr.m) && d_is_zero(dci.m))) {
             FE Xrfe = m ? Zfe[rm].re : fe_make(0.0, 0);
@@ -638,12 +647,14 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
             if (deriv_underflow) {
                 fe_deriv_underflow(zmrfe, zmife, SJ, jr, ji, invSJd);
             } else {
-                double a = 2.0 * (zmr * jr - zmi * ji) + invSJd;
-                double b = 2.0 * (zmr * ji + zmi * jr);
+                double a = d_twice(zmr * jr - zmi * ji) + invSJd;
+                double b = d_twice(zmr * ji + zmi * jr);
                 jr = a;
                 ji = b;
-                double jm2 = jr * jr + ji * ji;
-                if (jm2 > 1e16 || (jm2 > 0.0 && jm2 < 1e-16)) {
+                const unsigned hj = umax_(hi_abs(jr), hi_abs(ji));
+                double jm2 = 1.0;
+                if (hj < kFeWLo || hj >= kFeWHi) jm2 = jr * jr + ji * ji;
+                if (d_abs_less(1e16, jm2) || (d_abs_less(jm2, 1e-16) && !d_is_zero(jm2))) {
                     FE jmag = fe_sqrt(fe_from(jm2));
                     SJ = fe_mul(SJ, jmag);
                     double inv = 1.0 / fe_to_double(jmag);
@@ -656,11 +667,26 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
         X = m ? Z[rm] : make_double2(0.0, 0.0);
         Xr = X.x;
         Xi = X.y;
-        double zr = Xr + s * wr, zi = Xi + s * wi;
+        swr = s * wr;
+        swi = s * wi;
+        const double zr = Xr + swr, zi = Xi + swi;
+        oc.push(zr, zi);
+        // A common iteration: |z| between 1e-4 and the bailout and at least twice
+        // |dz|'s larger part (|z|^2 >= 4 max^2 > |dz|^2: no rebase), |w| in its
+        // window, the reference not at its end, and no interior test due.
+        const unsigned hz = umax_(hi_abs(zr), hi_abs(zi)), hw = umax_(hi_abs(wr), hi_abs(wi)), hs = umax_(hi_abs(swr), hi_abs(swi));
+        if (hz >= kFeNearWord && hz < p.esc_word && hz >= hs + 0x00100000u && hw >= kFeWLo && hw < kFeWHi && (per || m < reflen)) {
+            if (!detect) continue;
+            if (conf_P <= 0) {
+                if ((iter & 15) != 0 || conf_giveup >= 3) continue;
+                // z against the saved one: with a part 2^-27 of |z|'s larger part
+                // apart, |z - zs|^2 >= 5.5e-17 max^2 > 9e-18 2 max^2
+                if (iter - save_iter < period_win && umax_(hi_abs(zr - zsr), hi_abs(zi - zsi)) + 0x01b00000u >= hz && d_abs_less(p.interior_eps2, 1e-17)) continue;
+            }
+        }
         double zrad = zr * zr + zi * zi;
         const double wmag2 = wr * wr + wi * wi;
         bool keep = true;
-        oc.push(zr, zi);
         if (d_abs_less(g.ESC2, zrad)) { // zrad > ESC2
             o.n = iter;
             o.state = 1;
@@ -763,7 +789,10 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
                 keep = false;
             }
         }
-        if (keep) wm2_known = wmag2;
+        if (!keep) {
+            swr = s * wr;
+            swi = s * wi;
+        }
     }
     o.value = oc.interior();
     o.state = 2;
@@ -815,17 +844,10 @@ __device__ PixOut pixel_fe_nobla(const DeviceFrame& f, const FeParams& p, FE dcr
         const int current = index > mx_ref_it ? mx_ref_it : index;
         double2 zc = Z[current];
         double nwr, nwi;
-        if (p.fused) {
-            const double fR = (pr + pr) + (sd * wr);
-            const double fI = (pi + pi) + (sd * wi);
-            nwr = ((fR * wr) - (fI * wi)) + dr;
-            nwi = ((fR * wi) + (fI * wr)) + di;
-        } else {
-            const double sqR = (wr * wr) - (wi * wi), sqI = 2.0 * (wr * wi);
-            const double lR = (pr * wr) - (pi * wi), lI = (pr * wi) + (pi * wr);
-            nwr = ((2.0 * lR) + (sd * sqR)) + dr;
-            nwi = ((2.0 * lI) + (sd * sqI)) + di;
-        }
+        const double fR = (pr + pr) + (sd * wr);
+        const double fI = (pi + pi) + (sd * wi);
+        nwr = ((fR * wr) - (fI * wi)) + dr;
+        nwi = ((fR * wi) + (fI * wr)) + di;
         const double aR = zc.x + (sd * nwr), aI = zc.y + (sd * nwi);
         double actual = (aR * aR) + (aI * aI);
         double delta = (nwr * nwr) + (nwi * nwi);
@@ -1304,7 +1326,9 @@ cudaError_t launch_fp64_pass(const DeviceFrame& f, const Fp64Params& p, int bloc
     }
     return cudaGetLastError();
 }
-cudaError_t launch_fe_pass(const DeviceFrame& f, const FeParams& p, int blocks, int threads, cudaStream_t st) {
+cudaError_t launch_fe_pass(const DeviceFrame& f, const FeParams& fp, int blocks, int threads, cudaStream_t st) {
+    FeParams p = fp;
+    p.esc_word = direct_escape_word(p.g.ESC2);
     switch (p.g.oc) {
     case 0: k_fe_pass<0><<<blocks, threads, 0, st>>>(f, p); break;
     case kOcStripe: k_fe_pass<kOcStripe><<<blocks, threads, 0, st>>>(f, p); break;
