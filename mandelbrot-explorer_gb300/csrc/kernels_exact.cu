@@ -1,9 +1,7 @@
 // Exact-form CUDA passes of the perturbation renderer (compiled with
 // -fmad=false so that every double operation below is the IEEE operation the
 // reference executes, in the reference's order). Each kernel is persistent:
-// every thread pulls sample indices from a global work counter, so lanes whose
-// pixel finished are refilled immediately (the GPU form of the reference's
-// AVX2 lane refill, mp.cpp:416-532) instead of idling behind slow lanes.
+// every warp pulls its next samples from a global work counter (warp_take).
 //
 // Reference: cbotx/Mandelbrot-Explorer src/engine/mandel_perturbation.cpp
 // ("mp.cpp"); the per-pixel semantics are those of its scalar loops.
@@ -23,6 +21,24 @@ __device__ __forceinline__ int sample_index(const FrameGeom& g, const int* a) { 
 __device__ __forceinline__ void entry_key(const PixelSet& px, int i, int* a) { entry_coords(px, i, a); }
 
 __device__ __forceinline__ bool cancelled(const DeviceFrame& f) { return f.cancel && *f.cancel; }
+
+// The warp's next samples, taken together: the first of `lanes` consecutive
+// entries (lane k takes entry + k), or -1 when the work is done or cancelled.
+// Called by the warp's low `lanes` lanes, which so start every sample in step:
+// lanes that fetch one by one drift apart for good and the warp then executes
+// the loop once per drifted group (the 1e-300 frame's exact form cost twice as
+// much per sample at 1920x1080, 35 samples a lane, as at 480x270, one a lane).
+__device__ __forceinline__ int warp_take(const DeviceFrame& f, int n, int lanes) {
+    const unsigned mask = lanes >= 32 ? 0xffffffffu : (1u << lanes) - 1u;
+    __syncwarp(mask);
+    int base = -1;
+    // (plain read first: warps past the end leave without an atomic)
+    if ((threadIdx.x & 31u) == 0 && !cancelled(f) && (int)*(volatile unsigned int*)&f.ctr->next < n) {
+        base = (int)atomicAdd(&f.ctr->next, (unsigned)lanes);
+        if (base >= n) base = -1;
+    }
+    return __shfl_sync(mask, base, 0);
+}
 
 __device__ __forceinline__ double smooth_value(int n, double zrad) {
     return (double)n - log(log(zrad) / 2 / kLn2) / kLn2;
@@ -76,9 +92,10 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
     unsigned long long n_steps = 0, n_bla = 0, n_skip = 0, n_eff = 0;
     unsigned int n_int = 0;
     for (;;) {
-        if (cancelled(f)) break;
-        int i = (int)atomicAdd(&f.ctr->next, 1u);
-        if (i >= f.px.n) break;
+        const int first = warp_take(f, f.px.n, 32);
+        if (first < 0) break;
+        const int i = first + (int)(threadIdx.x & 31u);
+        if (i >= f.px.n) continue;
         int arr[4];
         entry_key(f.px, i, arr);
         // Per-pixel dc (mp.cpp:2300-2315) from the host-built mpf spacing tables.
@@ -261,7 +278,7 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
             }
             ++j;
         }
-        if (outcome == 4) break;
+        if (outcome == 4) continue; // cancelled
         if (outcome == 0 && j >= g.mxit) outcome = 2;
         const int idx = sample_index(g, arr);
         if (outcome == 1) {
@@ -917,12 +934,12 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
     unsigned long long n_steps = 0, n_bla = 0, n_skip = 0, n_eff = 0;
     unsigned int n_int = 0;
     const int n = f.px.n_dev ? min((int)*f.px.n_dev, f.px.n) : f.px.n;
+    const int lanes = p.lanes_per_warp ? p.lanes_per_warp : 32;
     for (;;) {
-        if (cancelled(f)) break;
-        // plain read first: threads past the end leave without an atomic
-        if ((int)*(volatile unsigned int*)&f.ctr->next >= n) break;
-        int i = (int)atomicAdd(&f.ctr->next, 1u);
-        if (i >= n) break;
+        const int first = warp_take(f, n, lanes);
+        if (first < 0) break;
+        const int i = first + (int)(threadIdx.x & 31u);
+        if (i >= n) continue;
         int arr[4];
         entry_key(f.px, i, arr);
         // dc in floatexp (mp.cpp:2160-2163).
@@ -932,7 +949,7 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
         FE Dci = fe_mul_d(p.dyfe, py - p.ref_y);
         // (the no-BLA lane kernel has no orbit colourings, mp.cpp:2148)
         PixOut o = (OC == 0 && p.no_bla_kernel) ? pixel_fe_nobla(f, p, Dcr, Dci, n_steps) : pixel_fe<OC>(f, p, Dcr, Dci, n_steps, n_bla, n_skip);
-        if (o.state == 4) break;
+        if (o.state == 4) continue; // cancelled
         const int idx = sample_index(g, arr);
         // mp.cpp:2173-2183: EMPTY or cutoff-sensitive results go to the
         // arbitrary-precision recompute, flagged here for the host.
@@ -1116,9 +1133,10 @@ __global__ void __launch_bounds__(128) k_julia(DeviceFrame f, JuliaParams p) {
     unsigned int n_int = 0;
     const int n = g.W * g.H;
     for (;;) {
-        if (cancelled(f)) break;
-        const int s = (int)atomicAdd(&f.ctr->next, 1u);
-        if (s >= n) break;
+        const int first = warp_take(f, n, 32);
+        if (first < 0) break;
+        const int s = first + (int)(threadIdx.x & 31u);
+        if (s >= n) continue;
         const int i = s / g.W, j = s - i * g.W;
         const double imag = p.z0i + p.dy * i;
         int nout = -1;
@@ -1148,9 +1166,10 @@ __global__ void __launch_bounds__(128) k_shallow(DeviceFrame f, ShallowParams p)
     unsigned long long n_eff = 0, n_steps = 0;
     unsigned int n_int = 0;
     for (;;) {
-        if (cancelled(f)) break;
-        int i = (int)atomicAdd(&f.ctr->next, 1u);
-        if (i >= f.px.n) break;
+        const int first = warp_take(f, f.px.n, 32);
+        if (first < 0) break;
+        const int i = first + (int)(threadIdx.x & 31u);
+        if (i >= f.px.n) continue;
         int arr[4];
         entry_key(f.px, i, arr);
         double cr, ci;
