@@ -14,9 +14,12 @@
 //     is iterated again by the plain loop (kDirectOpen);
 //   * counters are integers.
 // Six FP64 instructions a step instead of 34 in the shallow loop (14 in the
-// Julia loop), still bound by them. Measured: the whole set at 1280x720,
-// maxiter 5,000, 24.5 -> 5.7 ms a frame; a 160x120 Julia thumbnail, maxiter
-// 2,000, 1.00 -> 0.11 ms (its interior samples end at the first repeated z).
+// Julia loop). Measured with k_direct's packing (kernels_exact.cu): the whole
+// set at 1280x720, maxiter 5,000, 24.5 -> 2.3 ms a frame, of which the longest
+// sample's 5,000 steps alone take most; a 2560x1440 overlay image (dz/dc: 13
+// instructions a step) 107 -> 36.8 ms, bound by the FP64 unit; a 160x120 Julia
+// thumbnail, maxiter 2,000, 1.01 -> 0.11 ms (its interior samples end at the
+// first repeated z).
 // Host and device; compiled without FMA contraction.
 #pragma once
 #include "dfloat.cuh"
@@ -27,12 +30,6 @@ namespace mbx {
 
 MBX_HD unsigned hi_abs(double x) { return (unsigned)(dbits(x) >> 32) & 0x7fffffffu; }
 MBX_HD unsigned umax_(unsigned a, unsigned b) { return a > b ? a : b; }
-// x + x: an exponent increment for normal x with a normal result
-MBX_HD double twice(double x) {
-    const unsigned h = hi_abs(x);
-    if (h - 0x00100000u < 0x7fd00000u) return bitsd(dbits(x) + (1ull << 52));
-    return x + x;
-}
 MBX_HD unsigned float_bits(float x) {
 #ifdef __CUDA_ARCH__
     return __float_as_uint(x);
@@ -119,61 +116,124 @@ struct InteriorTrack {
     }
 };
 
-enum DirectEnd { kDirectEscaped = 1, kDirectInterior = 2, kDirectOpen = 3 };
+// How a step leaves a sample.
+enum DirectEnd { kDirectRuns = 0, kDirectEscaped = 1, kDirectInterior = 2, kDirectOpen = 3 };
 
-struct DirectState {
-    double zr, zi, zrad;   // the escaped z and |z|^2
-    double dcr, dci;       // dz/dc (DERIV)
-    int n;                 // iterations taken
-};
-
-// Iterate z from c at most until n reaches mxit (n starts at 1). LANE: the
-// reference's lane kernel (mp.cpp:416-532) takes a step before it looks at
-// maxiter and doubles the product zr zi; its scalar loop (mp.cpp:330-399) looks
-// first and doubles zr. DERIV: dz/dc as well. visit(zr, zi) sees every z.
-template <bool LANE, bool DERIV, class Visit>
-MBX_HD int direct_iterate(double cr, double ci, int mxit, double esc2, unsigned esc_word, DirectState& s, Visit&& visit) {
-    double zr = cr, zi = ci, dcr = 1, dci = 0;
-    s.n = 1;
-    if (!LANE && mxit <= 1) return kDirectInterior;
-    unsigned hm = umax_(hi_abs(zr), hi_abs(zi));
-    if (hm >= kDirectFarWord || hm < kDirectTinyWord || !direct_trackable(esc2)) return kDirectOpen;
+// One sample of z -> z^2 + c from z = c. LANE: the reference's lane kernel
+// (mp.cpp:416-532) takes a step before it looks at maxiter and doubles the
+// product zr zi; its scalar loop (mp.cpp:330-399) looks first and doubles zr.
+// DERIV: dz/dc as well. visit(zr, zi, zr^2, zi^2) sees every z.
+template <bool LANE, bool DERIV>
+struct DirectLane {
+    double zr, zi, x2, y2, cr, ci;
+    double dcr, dci;
     InteriorTrack track;
-    double x2 = zr * zr, y2 = zi * zi;
-    for (int n = 1;;) {
+    int n; // iterations taken plus one; at the escape, the escape iteration
+    unsigned hm;
+
+    MBX_HD int start(double c_re, double c_im, int mxit, double esc2) {
+        zr = cr = c_re;
+        zi = ci = c_im;
+        dcr = 1.0;
+        dci = 0.0;
+        n = 1;
+        track = InteriorTrack();
+        if (!LANE && mxit <= 1) return kDirectInterior;
+        hm = umax_(hi_abs(zr), hi_abs(zi));
+        if (hm >= kDirectFarWord || hm < kDirectTinyWord || !direct_trackable(esc2)) return kDirectOpen;
+        x2 = zr * zr;
+        y2 = zi * zi;
+        return kDirectRuns;
+    }
+    // One step, without its tests: true when one of them may apply (one branch a
+    // step: the tests' own would hold up a lone sample's chain). hm: the larger
+    // part's high word.
+    template <class Visit>
+    MBX_HD bool advance(int mxit, unsigned esc_word, Visit&& visit) {
+        const double s = x2 - y2, m = LANE ? d_twice(zr * zi) : d_twice(zr) * zi;
         track.step(x2, y2);
         if (DERIV) {
-            const double t = twice(dcr * zr - dci * zi) + 1.0;
-            dci = twice(dcr * zi + dci * zr);
+            const double t = d_twice(dcr * zr - dci * zi) + 1.0;
+            dci = d_twice(dcr * zi + dci * zr);
             dcr = t;
         }
-        const double nzi = (LANE ? twice(zr * zi) : twice(zr) * zi) + ci;
-        zr = (x2 - y2) + cr;
-        zi = nzi;
+        zr = s + cr;
+        zi = m + ci;
         x2 = zr * zr;
         y2 = zi * zi;
         visit(zr, zi, x2, y2);
         hm = umax_(hi_abs(zr), hi_abs(zi));
-        if (hm >= esc_word) {
-            const double zrad = x2 + y2;
-            if (d_abs_less(esc2, zrad)) { // zrad > esc2
-                s.zr = zr;
-                s.zi = zi;
-                s.zrad = zrad;
-                s.dcr = dcr;
-                s.dci = dci;
-                s.n = n + 1;
-                return kDirectEscaped;
-            }
-        }
+        ++n;
+        return hm >= esc_word || hm < kDirectTinyWord || track.e <= -30 || n >= mxit;
+    }
+    // The tests of that step, in the reference's order.
+    MBX_HD int resolve(int mxit, double esc2, unsigned esc_word) const {
+        if (hm >= esc_word && d_abs_less(esc2, x2 + y2)) return kDirectEscaped; // |z|^2 > esc2
         if (track.e <= -30) {
-            const int b = track.below(n);
+            const int b = track.below(n - 1);
             if (b) return b == 1 ? kDirectInterior : kDirectOpen;
         }
-        if (++n >= mxit) return kDirectInterior;
-        if (hm < kDirectTinyWord) return kDirectOpen; // |z|^2 near split2f's floor
+        if (n >= mxit) return kDirectInterior;
+        return hm < kDirectTinyWord ? kDirectOpen : kDirectRuns; // (|z|^2 near split2f's floor)
     }
-}
+    template <class Visit>
+    MBX_HD int step(int mxit, double esc2, unsigned esc_word, Visit&& visit) {
+        return advance(mxit, esc_word, visit) ? resolve(mxit, esc2, esc_word) : kDirectRuns;
+    }
+};
+
+// One Julia sample of z -> z^2 + c (solveJuliaShallowSimdList, mp.cpp:534-636;
+// D' = 2 z D from D_0 = 1 under DERIV). A z that repeats an earlier one bit for
+// bit cycles for ever: the orbit never escapes (Brent's doubling window).
+template <bool DERIV>
+struct JuliaLane {
+    double zr, zi, x2, y2;
+    double dcr, dci; // D
+    uint64_t sr, si;
+    int n, next, win; // n: iterations taken
+
+    MBX_HD int start(double z_re, double z_im, double esc2) {
+        zr = z_re;
+        zi = z_im;
+        x2 = zr * zr;
+        y2 = zi * zi;
+        dcr = 1.0;
+        dci = 0.0;
+        n = 0;
+        sr = si = ~0ull; // (a NaN: no finite z equals it)
+        next = win = 8;
+        return d_abs_less(esc2, x2 + y2) ? kDirectEscaped : kDirectRuns;
+    }
+    // (as DirectLane::advance and resolve; the repeat is looked for on one low word)
+    MBX_HD bool advance(double cr, double ci, int mxit, unsigned esc_word) {
+        const double s = x2 - y2, m = zr * zi;
+        if (DERIV) {
+            const double t = d_twice(dcr * zr - dci * zi);
+            dci = d_twice(dcr * zi + dci * zr);
+            dcr = t;
+        }
+        zr = s + cr;
+        zi = d_twice(m) + ci;
+        x2 = zr * zr;
+        y2 = zi * zi;
+        ++n;
+        return umax_(hi_abs(zr), hi_abs(zi)) >= esc_word || n >= mxit || n == next || (unsigned)dbits(zr) == (unsigned)sr;
+    }
+    MBX_HD int resolve(int mxit, double esc2) {
+        if (d_abs_less(esc2, x2 + y2)) return kDirectEscaped;
+        if (n >= mxit || (dbits(zr) == sr && dbits(zi) == si)) return kDirectInterior;
+        if (n == next) {
+            sr = dbits(zr);
+            si = dbits(zi);
+            next = n > (1 << 29) ? 0x7fffffff : n + win;
+            win += win > (1 << 29) ? 0 : win;
+        }
+        return kDirectRuns;
+    }
+    MBX_HD int step(double cr, double ci, int mxit, double esc2, unsigned esc_word) {
+        return advance(cr, ci, mxit, esc_word) ? resolve(mxit, esc2) : kDirectRuns;
+    }
+};
 
 // OrbitTrap over the direct iteration's finite z: the same minima, with the
 // comparisons on bit patterns and |z|^2, sqrt |z|^2 in FP64 only where a
@@ -221,56 +281,5 @@ struct DirectTrap {
         }
     }
 };
-
-// The Julia iteration z -> z^2 + c from z (solveJuliaShallowSimdList,
-// mp.cpp:534-636; D' = 2 z D from D_0 = 1 under DERIV). A z that repeats an
-// earlier one bit for bit cycles for ever: the orbit never escapes (Brent's
-// doubling window). Returns 1 escaped, 2 not.
-template <bool DERIV>
-MBX_HD int julia_iterate(double zr, double zi, double cr, double ci, int mxit, double esc2, unsigned esc_word, DirectState& s) {
-    double dr = 1.0, di = 0.0;
-    double x2 = zr * zr, y2 = zi * zi;
-    s.zr = zr;
-    s.zi = zi;
-    s.zrad = x2 + y2;
-    s.dcr = 1.0;
-    s.dci = 0.0;
-    s.n = 0;
-    if (d_abs_less(esc2, s.zrad)) return kDirectEscaped;
-    uint64_t sr = ~0ull, si = ~0ull; // (a NaN: equals no finite z)
-    int next = 8, win = 8;
-    for (int n = 0;;) {
-        if (DERIV) {
-            const double t = twice(dr * zr - di * zi);
-            di = twice(dr * zi + di * zr);
-            dr = t;
-        }
-        const double nzi = twice(zr * zi) + ci;
-        zr = (x2 - y2) + cr;
-        zi = nzi;
-        x2 = zr * zr;
-        y2 = zi * zi;
-        ++n;
-        if (umax_(hi_abs(zr), hi_abs(zi)) >= esc_word) {
-            const double zrad = x2 + y2;
-            if (d_abs_less(esc2, zrad)) {
-                s.zr = zr;
-                s.zi = zi;
-                s.zrad = zrad;
-                s.dcr = dr;
-                s.dci = di;
-                s.n = n;
-                return kDirectEscaped;
-            }
-        }
-        if (n >= mxit || (dbits(zr) == sr && dbits(zi) == si)) return kDirectInterior;
-        if (n == next) {
-            sr = dbits(zr);
-            si = dbits(zi);
-            next = n > (1 << 29) ? 0x7fffffff : n + win;
-            win += win > (1 << 29) ? 0 : win;
-        }
-    }
-}
 
 } // namespace mbx

@@ -2394,10 +2394,10 @@ int Engine::render_julia(mpf_ptr z_re, mpf_ptr z_im, mpf_ptr scale, const char* 
             mpf_add(c0_im_, c0_im_, dw);
         }
     }
-    JuliaParams p;
+    ShallowParams p{};
     p.g = geom();
-    p.z0r = mpf_ld(c0_re_);
-    p.z0i = mpf_ld(c0_im_);
+    p.c0r = mpf_ld(c0_re_);
+    p.c0i = mpf_ld(c0_im_);
     p.dx = mpf_ld(dx_);
     p.dy = mpf_ld(dy_);
     p.cr = mpf_ld(cr);
@@ -2405,9 +2405,15 @@ int Engine::render_julia(mpf_ptr z_re, mpf_ptr z_im, mpf_ptr scale, const char* 
     const int n = W_ * H_;
     cudaMemsetAsync(dctr_, 0, sizeof(Counters), st_);
     DeviceFrame f = frame_view();
+    f.px = PixelSet();
+    f.px.n = n;
+    f.px.grid_w = W_;
+    f.px.grid_h = H_;
+    f.px.grid_step = 1;
+    f.px.skip_i = f.px.skip_j = -1;
     const double t0 = now_ms();
     cudaEventRecord(ev0_, st_);
-    cudaError_t e = launch_julia(f, p, std::min((n + 127) / 128, nsm_ * 8), 128, st_);
+    cudaError_t e = launch_julia(f, p, nsm_, st_);
     cudaEventRecord(ev1_, st_);
     ++stats_.kernel_launches;
     ++stats_.passes;
@@ -2447,7 +2453,7 @@ int Engine::render_shallow(volatile float* progress) {
     DeviceFrame f = frame_view();
     f.px = g;
     const double t0 = now_ms();
-    cudaError_t e = launch_shallow(f, p, std::min((g.n + 127) / 128, nsm_ * 8), 128, st_);
+    cudaError_t e = launch_shallow(f, p, nsm_, st_);
     ++stats_.kernel_launches;
     ++stats_.passes;
     if (e != cudaSuccess) return fail_cuda("shallow launch", e);
@@ -2490,7 +2496,7 @@ int Engine::shallow_samples(const std::vector<uint64_t>& samples) {
     DeviceFrame f = frame_view();
     f.px = g;
     const double t0 = now_ms();
-    cudaError_t e = launch_shallow(f, p, std::min((n + 127) / 128, nsm_ * 8), 128, st_);
+    cudaError_t e = launch_shallow(f, p, nsm_, st_);
     ++stats_.kernel_launches;
     ++stats_.passes;
     if (e != cudaSuccess) return fail_cuda("shallow ss launch", e);

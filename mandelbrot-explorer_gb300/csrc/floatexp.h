@@ -59,7 +59,8 @@ MBX_HD bool d_le_zero(double x) {
     const uint64_t u = dbits(x);
     return (u << 1) == 0 || ((u >> 63) != 0 && (u & 0x7fffffffffffffffull) <= 0x7ff0000000000000ull);
 }
-// x + x, exactly as the FP64 add rounds it, on the bit pattern for finite x
+// x + x, exactly as the FP64 add rounds it, on the bit pattern. (No FP64 add even
+// for the rare cases: the compiler would execute it beside the common one.)
 MBX_HD double d_twice(double x) {
     const uint64_t b = dbits(x);
     const uint64_t e = (b >> 52) & 0x7ff;
@@ -67,7 +68,7 @@ MBX_HD double d_twice(double x) {
     if (e == 0) // zero or subnormal: the magnitude shifts (a carry into the exponent gives the normal result)
         return bitsd((b & 0x8000000000000000ull) | ((b & 0x7fffffffffffffffull) << 1));
     if (e == 0x7fe) return bitsd((b & 0x8000000000000000ull) | 0x7ff0000000000000ull); // overflows to infinity
-    return x + x; // infinity, NaN
+    return x; // infinity, NaN
 }
 
 // frexp: x = r * 2^e with 0.5 <= |r| < 1; zero, inf and nan return x with e = 0.

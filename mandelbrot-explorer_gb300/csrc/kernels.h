@@ -179,20 +179,15 @@ struct FeParams {
     int lanes_per_warp = 0;  // exact-form leftovers: lanes of each warp that take samples (0: all 32)
 };
 
-// Shallow direct loop (mp.cpp:330-532).
+// The direct loops: shallow frames (mp.cpp:330-532) and Julia frames
+// (Mandel::ComputeJulia, mp.cpp:992-1044: c0 is the lower-left z0, cr, ci the
+// fixed c).
 struct ShallowParams {
     FrameGeom g;
-    double c0r, c0i, dx, dy;
+    double c0r, c0i, dx, dy; // lower-left sample and spacings (mpf_get_ld)
     int simd_semantics;      // 1: lane-refill kernel (float result), 0: floatPointCompute
-    unsigned esc_word = 0;   // direct_escape_word(g.ESC2), set by launch_shallow
-};
-
-// Julia frames (Mandel::ComputeJulia, mp.cpp:992-1044): z0 = c0 + (dx j, dy i).
-struct JuliaParams {
-    FrameGeom g;
-    double z0r, z0i, dx, dy; // lower-left sample and spacings (mpf_get_ld)
-    double cr, ci;           // the fixed c
-    unsigned esc_word = 0;   // direct_escape_word(g.ESC2), set by launch_julia
+    double cr = 0.0, ci = 0.0;
+    unsigned esc_word = 0;   // direct_escape_word(g.ESC2), set by the launchers
 };
 
 struct DeviceFrame {
@@ -210,8 +205,8 @@ struct DeviceFrame {
 cudaError_t launch_fill(float* iter, float* normal, int32_t* escN, size_t n, cudaStream_t st);
 cudaError_t launch_fp64_pass(const DeviceFrame& f, const Fp64Params& p, int blocks, int threads, cudaStream_t st);
 cudaError_t launch_fe_pass(const DeviceFrame& f, const FeParams& p, int blocks, int threads, cudaStream_t st);
-cudaError_t launch_shallow(const DeviceFrame& f, const ShallowParams& p, int blocks, int threads, cudaStream_t st);
-cudaError_t launch_julia(const DeviceFrame& f, const JuliaParams& p, int blocks, int threads, cudaStream_t st);
+cudaError_t launch_shallow(const DeviceFrame& f, const ShallowParams& p, int nsm, cudaStream_t st);
+cudaError_t launch_julia(const DeviceFrame& f, const ShallowParams& p, int nsm, cudaStream_t st);
 cudaError_t launch_bla_build(const double2* Z, const double2* D, int reflen, double eps, double dcmax, bool ede,
                              double* r2, double4* ab, double4* ce, const int* off, const int* size, int nlev,
                              unsigned long long* rmax2_bits, cudaStream_t st);

@@ -9,6 +9,8 @@
 #include "kernels.h"
 #include "orbit_color.h"
 
+#include <type_traits>
+
 namespace mbx {
 
 static constexpr double kLn2 = 0x1.62e42fefa39efp-1; // log(2.0), correctly rounded
@@ -977,12 +979,17 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
 }
 
 // ---------------------------------------------------------------------------
-// Shallow direct loop: floatPointCompute (mp.cpp:330-399) and the lane-refill
-// kernel's per-lane arithmetic (mp.cpp:416-532). The plain loops below, with the
-// interior test's derivative in FP64, take only the samples that
-// direct_iterate (direct_loop.cuh) leaves open.
+// The direct loops: shallow frames (floatPointCompute, mp.cpp:330-399, and the
+// lane-refill kernel's per-lane arithmetic, mp.cpp:416-532) and Julia frames
+// (ComputeJulia, mp.cpp:992-1041). The plain loops here, with the interior
+// test's derivative in FP64, take only the samples that direct_loop.cuh leaves
+// open.
+struct DirectEndState {
+    double zr, zi, zrad, dcr, dci;
+    int n;
+};
 template <int OC>
-__device__ __noinline__ int shallow_scalar_plain(double c_re, double c_im, int mxit, const FrameGeom& g, DirectState& s, OrbitColor<OC>& oc) {
+__device__ __noinline__ int shallow_scalar_plain(double c_re, double c_im, int mxit, const FrameGeom& g, DirectEndState& s, OrbitColor<OC>& oc) {
     double z_re = c_re, z_im = c_im, d_re = 2, d_im = 0, dc_re = 1, dc_im = 0, tmp;
     const bool deriv = g.ede || g.deovl || g.normal;
     oc.init(); // mp.cpp:347-369
@@ -1002,7 +1009,7 @@ __device__ __noinline__ int shallow_scalar_plain(double c_re, double c_im, int m
         oc.push(z_re, z_im);
         tmp = z_re * z_re + z_im * z_im;
         if (tmp > g.ESC2) {
-            s = DirectState{z_re, z_im, tmp, dc_re, dc_im, i + 1};
+            s = DirectEndState{z_re, z_im, tmp, dc_re, dc_im, i + 1};
             return kDirectEscaped;
         }
         tmp = d_re * d_re + d_im * d_im;
@@ -1012,7 +1019,7 @@ __device__ __noinline__ int shallow_scalar_plain(double c_re, double c_im, int m
     return kDirectInterior;
 }
 
-__device__ __noinline__ int shallow_lane_plain(double cr, double ci, int mxit, const FrameGeom& g, DirectState& s) {
+__device__ __noinline__ int shallow_lane_plain(double cr, double ci, int mxit, const FrameGeom& g, DirectEndState& s) {
     double zr = cr, zi = ci, dr = 2, di = 0, dcr = 1, dci = 0;
     for (int n = 1;; ++n) {
         double ndr = 2.0 * ((dr * zr) - (di * zi));
@@ -1030,187 +1037,352 @@ __device__ __noinline__ int shallow_lane_plain(double cr, double ci, int mxit, c
         double zrad = (zr * zr) + (zi * zi);
         double dmag = (dr * dr) + (di * di);
         if (zrad > g.ESC2) {
-            s = DirectState{zr, zi, zrad, dcr, dci, n + 1};
+            s = DirectEndState{zr, zi, zrad, dcr, dci, n + 1};
             return kDirectEscaped;
         }
         if (dmag < 1e-9 || n + 1 >= mxit) return kDirectInterior;
     }
 }
 
-// The distance sqrt(zrad) log(zrad) / |dz/dc|.
-__device__ __forceinline__ double direct_distance(const DirectState& s) {
-    return sqrt(s.zrad) * log(s.zrad) / sqrt(s.dcr * s.dcr + s.dci * s.dci);
-}
-// The lane kernel's value (float): the smooth count, or the distance under EDE; -2 interior.
-__device__ float shallow_lane(double cr, double ci, int mxit, const FrameGeom& g, unsigned esc_word, int* nout) {
-    DirectState s;
-    auto none = [](double, double, double, double) {};
-    int st = g.ede ? direct_iterate<true, true>(cr, ci, mxit, g.ESC2, esc_word, s, none) : direct_iterate<true, false>(cr, ci, mxit, g.ESC2, esc_word, s, none);
-    if (st == kDirectOpen) st = shallow_lane_plain(cr, ci, mxit, g, s);
-    if (st == kDirectInterior) return -2.0f;
-    *nout = s.n;
-    if (g.ede) return (float)direct_distance(s);
-    return (float)smooth_value(s.n, s.zrad);
-}
-
-// The stripe average of an escaped sample: its last kStripeWindow terms, from
-// the orbit iterated once more (the trigonometry of the other iterations, and
-// of every interior sample, is never formed; with at most a window of
-// iterations the sums are those of the reference operation for operation).
-__device__ __noinline__ float shallow_stripe(double cr, double ci, const DirectState& s, double ER) {
+// The stripe average of an escaped sample: the terms of its last
+// kStripeWindow iterates, from the orbit iterated again from z_k = (zr, zi) (the
+// trigonometry of the other iterations, and of every interior sample, is never
+// formed; with at most a window of iterations the sums are the reference's).
+__device__ __noinline__ float shallow_stripe(double cr, double ci, double zr, double zi, int k, int n, double zrad, double ER) {
     StripeTail tail;
     tail.init();
-    double zr = cr, zi = ci, x2 = zr * zr, y2 = zi * zi;
-    const int first = s.n - kStripeWindow;
-    for (int k = 1; k < s.n; ++k) {
-        const double nzi = twice(zr) * zi + ci;
+    double x2 = zr * zr, y2 = zi * zi;
+    const int first = n - kStripeWindow;
+    for (++k; k < n; ++k) {
+        const double nzi = d_twice(zr) * zi + ci;
         zr = (x2 - y2) + cr;
         zi = nzi;
         x2 = zr * zr;
         y2 = zi * zi;
         if (k >= first) tail.push(zr, zi);
     }
-    return tail.value(s.zrad, ER);
+    return tail.value(zrad, ER);
 }
+// Where to start again: the sample keeps its z of the last two multiples of the
+// window; the earlier one lies a window or more before the last iterate z_(n-1).
+struct StripeMark {
+    double zr, zi, nr, ni;
+    __device__ void visit(int k, double r, double i) {
+        if ((k & (kStripeWindow - 1)) == 0) {
+            zr = nr;
+            zi = ni;
+            nr = r;
+            ni = i;
+        }
+    }
+};
+__device__ __forceinline__ int stripe_mark(int n) { return ((n - 1) & ~(kStripeWindow - 1)) - kStripeWindow; } // (<= 0: from c)
 
-// floatPointCompute's value, its normal angle or overlay distance in *nrm.
-template <int OC>
-__device__ double shallow_scalar(double c_re, double c_im, int mxit, const FrameGeom& g, unsigned esc_word, double* nrm, int* nout) {
-    const bool deriv = g.ede || g.deovl || g.normal;
-    DirectState s;
-    int st;
-    DirectTrap trap;
-    if (OC & kOcTrap) {
-        trap.init();
-        auto visit = [&](double zr, double zi, double x2, double y2) { trap.push(zr, zi, x2, y2); };
-        st = deriv ? direct_iterate<false, true>(c_re, c_im, mxit, g.ESC2, esc_word, s, visit) : direct_iterate<false, false>(c_re, c_im, mxit, g.ESC2, esc_word, s, visit);
+// Which loop a direct pass runs, and what its samples are.
+enum DirectForm { kFormLane, kFormScalar, kFormJulia };
+
+// The sample's c (z0 of a Julia frame) of pass entry i.
+__device__ __forceinline__ void direct_c(const DeviceFrame& f, const ShallowParams& p, const int* arr, double& cr, double& ci) {
+    if (arr[2] == 0 && arr[3] == 0 && !f.px.keys) {
+        ci = p.c0i + p.dy * arr[0];
+        cr = p.c0r + p.dx * arr[1];
     } else {
-        auto visit = [](double, double, double, double) {};
-        st = deriv ? direct_iterate<false, true>(c_re, c_im, mxit, g.ESC2, esc_word, s, visit) : direct_iterate<false, false>(c_re, c_im, mxit, g.ESC2, esc_word, s, visit);
+        cr = p.c0r + p.dx * arr[1] + p.dx * arr[3] / p.g.sub;
+        ci = p.c0i + p.dy * arr[0] + p.dy * arr[2] / p.g.sub;
     }
-    OrbitColor<OC & kOcTrap> oc; // the trap; a stripe average is formed at the escape
-    if (st == kDirectOpen) st = shallow_scalar_plain<OC & kOcTrap>(c_re, c_im, mxit, g, s, oc);
-    else trap.give(oc);
-    if (st == kDirectInterior) return oc.interior();
-    *nout = s.n;
-    if (g.ede) return direct_distance(s);
-    const double mu = smooth_value(s.n, s.zrad);
-    if (g.normal) { // mp.cpp:375-378
-        if (nrm) *nrm = atan2(s.zi, s.zr) - atan2(s.dci, s.dcr);
-    } else if (g.deovl) {
-        if (nrm) *nrm = direct_distance(s);
-    } else if (OC & kOcTrap) { // mp.cpp:383-389
-        return oc.escaped(mu, s.zrad, g.ER);
-    } else if (OC & kOcStripe) {
-        return shallow_stripe(c_re, c_im, s, g.ER);
-    }
-    return mu;
 }
 
-// One Julia sample: z0 the sample, c fixed (julia_iterate). nout: escape index
-// (0 when z0 is already outside), -1 interior.
-__device__ float julia_lane(double zr, double zi, double cr, double ci, int mxit, const FrameGeom& g, unsigned esc_word, int* nout) {
-    DirectState s;
-    const int st = g.ede ? julia_iterate<true>(zr, zi, cr, ci, mxit, g.ESC2, esc_word, s) : julia_iterate<false>(zr, zi, cr, ci, mxit, g.ESC2, esc_word, s);
-    *nout = -1;
-    if (st == kDirectInterior) return -2.0f;
-    *nout = s.n;
-    if (g.ede) {
-        const double num = sqrt(s.zrad) * log(s.zrad);
-        if (s.n == 0) return (float)num;
-        const double denom = sqrt((s.dcr * s.dcr) + (s.dci * s.dci));
-        return denom > 0.0 ? (float)(num / denom) : 0.0f;
-    }
-    const double x = log(log(s.zrad) / 2 / kLn2) / kLn2;
-    return s.n == 0 ? (float)(-x) : (float)((double)s.n - x);
-}
+// A finished sample waiting for its value: the escape iteration (interior: -1),
+// z and |z|^2 there, and dz/dc or, under a trap, its minima (a, b, zr), under a
+// stripe average its mark (a, b).
+struct DirectDone {
+    double zrad, a, b, zr, zi;
+    int n, i;
+};
 
-// ComputeJulia's frame (mp.cpp:1019-1041): every sample of the grid, the EDE
-// value divided by (float)dx.
-__global__ void __launch_bounds__(128) k_julia(DeviceFrame f, JuliaParams p) {
+// The sample's value and outputs (mp.cpp:373-398, 1500-1515; Julia :1019-1041).
+template <int FORM, int OC>
+__device__ __forceinline__ void direct_write(const DeviceFrame& f, const ShallowParams& p, const DirectDone& d) {
     const FrameGeom& g = p.g;
-    unsigned long long n_eff = 0, n_steps = 0;
-    unsigned int n_int = 0;
-    const int n = g.W * g.H;
-    for (;;) {
-        const int first = warp_take(f, n, 32);
-        if (first < 0) break;
-        const int s = first + (int)(threadIdx.x & 31u);
-        if (s >= n) continue;
-        const int i = s / g.W, j = s - i * g.W;
-        const double imag = p.z0i + p.dy * i;
-        int nout = -1;
-        float v = julia_lane(p.z0r + p.dx * j, imag, p.cr, p.ci, g.mxit, g, p.esc_word, &nout);
-        if (g.ede && v >= 0.0f) v /= (float)p.dx;
-        f.out.iter[s] = v;
-        if (f.out.escN) f.out.escN[s] = nout;
-        if (nout >= 0) {
-            n_eff += (unsigned long long)nout;
-            n_steps += (unsigned long long)nout;
-        } else {
-            n_eff += (unsigned long long)g.mxit;
-            n_steps += (unsigned long long)g.mxit;
-            ++n_int;
-        }
-    }
-    atomicAdd(&f.ctr->effective_iters, n_eff);
-    atomicAdd(&f.ctr->steps, n_steps);
-    atomicAdd(&f.ctr->interior, n_int);
-}
-
-// Base pass (mp.cpp:1483-1519) in grid mode, or adaptive-SS sub-samples
-// (mp.cpp:1920-1969) from a key list.
-template <int OC>
-__global__ void __launch_bounds__(128) k_shallow(DeviceFrame f, ShallowParams p) {
-    const FrameGeom& g = p.g;
-    unsigned long long n_eff = 0, n_steps = 0;
-    unsigned int n_int = 0;
-    for (;;) {
-        const int first = warp_take(f, f.px.n, 32);
-        if (first < 0) break;
-        const int i = first + (int)(threadIdx.x & 31u);
-        if (i >= f.px.n) continue;
-        int arr[4];
-        entry_key(f.px, i, arr);
-        double cr, ci;
-        if (arr[2] == 0 && arr[3] == 0 && !f.px.keys) {
-            ci = p.c0i + p.dy * arr[0];
-            cr = p.c0r + p.dx * arr[1];
-        } else {
-            cr = p.c0r + p.dx * arr[1] + p.dx * arr[3] / g.sub;
-            ci = p.c0i + p.dy * arr[0] + p.dy * arr[2] / g.sub;
-        }
-        const int idx = sample_index(g, arr);
-        int nout = -1;
-        double val;
-        if (OC == 0 && p.simd_semantics) { // (no orbit colourings in the lane kernel, mp.cpp:1459)
-            val = (double)shallow_lane(cr, ci, g.mxit, g, p.esc_word, &nout);
-            if (g.ede && val >= 0) val /= p.dx;
-            f.out.iter[idx] = (float)val;
-        } else {
-            double de = 0.0;
-            val = shallow_scalar<OC>(cr, ci, g.mxit, g, p.esc_word, &de, &nout);
-            if (g.normal) { // mp.cpp:1504-1507 (with EDE also set: the raw distance, angle 0)
-                f.out.iter[idx] = (float)val;
-                if (f.out.normal) f.out.normal[idx] = (float)de;
-            } else if (g.deovl) {
-                float v = (float)val;
-                f.out.iter[idx] = v;
-                if (f.out.normal) f.out.normal[idx] = (v < 0) ? 0.0f : (float)(de / p.dx);
-            } else { // the value is stored as float before the EDE division (mp.cpp:1512-1515)
-                float v = (float)val;
-                if (g.ede && v >= 0) v = (float)((double)v / p.dx);
-                f.out.iter[idx] = v;
+    int arr[4];
+    entry_key(f.px, d.i, arr);
+    const int idx = sample_index(g, arr);
+    const bool inside = d.n < 0;
+    if (FORM == kFormJulia) {
+        float v = -2.0f;
+        if (!inside) {
+            if (g.ede) {
+                const double num = sqrt(d.zrad) * log(d.zrad);
+                if (d.n == 0) {
+                    v = (float)num;
+                } else {
+                    const double denom = sqrt((d.a * d.a) + (d.b * d.b));
+                    v = denom > 0.0 ? (float)(num / denom) : 0.0f;
+                }
+                if (v >= 0.0f) v /= (float)p.dx;
+            } else {
+                const double x = log(log(d.zrad) / 2 / kLn2) / kLn2;
+                v = d.n == 0 ? (float)(-x) : (float)((double)d.n - x);
             }
         }
-        if (f.out.escN) f.out.escN[idx] = nout;
-        f.out.done[i] = 1;
-        if (nout > 0) {
-            n_eff += (unsigned long long)nout;
-            n_steps += (unsigned long long)nout;
+        f.out.iter[idx] = v;
+        if (f.out.escN) f.out.escN[idx] = d.n;
+        return;
+    }
+    double val = -2.0, de = 0.0;
+    if (OC & kOcTrap) {
+        if (inside || !(g.ede || g.normal || g.deovl)) { // (an escaped DE sample's value is not its trap's)
+            OrbitTrap t;
+            t.point2 = d.a;
+            t.cross = d.b;
+            t.circle = d.zr;
+            val = inside ? (double)t.value(0.0) : (double)t.value(smooth_value(d.n, d.zrad)); // mp.cpp:383-389
+        }
+    }
+    if (!inside && !((OC & kOcTrap) && !(g.ede || g.normal || g.deovl))) {
+        const bool distance = g.ede || (g.deovl && !g.normal);
+        const double dist = distance ? sqrt(d.zrad) * log(d.zrad) / sqrt(d.a * d.a + d.b * d.b) : 0.0;
+        if (g.ede) {
+            val = dist;
         } else {
-            n_eff += (unsigned long long)g.mxit;
-            ++n_int;
+            if (g.normal) de = atan2(d.zi, d.zr) - atan2(d.b, d.a); // mp.cpp:375-378
+            else if (g.deovl) de = dist;
+            if (OC == kOcStripe && !g.normal && !g.deovl) {
+                double cr, ci;
+                direct_c(f, p, arr, cr, ci);
+                const int k = stripe_mark(d.n);
+                val = k > 0 ? shallow_stripe(cr, ci, d.a, d.b, k, d.n, d.zrad, g.ER) : shallow_stripe(cr, ci, cr, ci, 0, d.n, d.zrad, g.ER);
+            } else {
+                val = smooth_value(d.n, d.zrad);
+            }
+        }
+    }
+    if (FORM == kFormLane) {
+        val = (double)(float)val;
+        if (g.ede && val >= 0) val /= p.dx;
+        f.out.iter[idx] = (float)val;
+    } else if (g.normal) { // mp.cpp:1504-1507 (with EDE also set: the raw distance, angle 0)
+        f.out.iter[idx] = (float)val;
+        if (f.out.normal) f.out.normal[idx] = (float)de;
+    } else if (g.deovl) {
+        float v = (float)val;
+        f.out.iter[idx] = v;
+        if (f.out.normal) f.out.normal[idx] = (v < 0) ? 0.0f : (float)(de / p.dx);
+    } else { // the value is stored as float before the EDE division (mp.cpp:1512-1515)
+        float v = (float)val;
+        if (g.ede && v >= 0) v = (float)((double)v / p.dx);
+        f.out.iter[idx] = v;
+    }
+    if (f.out.escN) f.out.escN[idx] = d.n;
+    f.out.done[d.i] = 1;
+}
+
+// The direct pass, persistent. Neighbouring samples differ widely in length (the
+// whole set at 1280x720: 43 steps a sample, 276 the longest of 32 neighbours), and
+// an FP64 warp instruction costs the same with one lane as with 32, so lanes are
+// kept full:
+//   * while samples are left, a warp steps its lanes in blocks of kDirectBlock
+//     and fetches new samples once kDirectRefill lanes are idle;
+//   * then the block's threads, few of them still iterating, are packed into as
+//     few warps as hold them, every kDirectRound steps (the samples left are
+//     the longest: without this they ran 6.6 to a warp);
+//   * a value costs over a hundred FP64 instructions (log, sqrt, divisions;
+//     atan2 and sin for a stripe average), so finished samples wait in shared
+//     memory until a warp has 32 and forms them in full (a stripe average's terms
+//     are as many as the orbit is long: short and long orbits wait apart).
+// Measured (1280x720 whole set / stripe average 601x399 with 3x3 supersampling /
+// 2560x1440 overlay image): one sample after the other per lane 5.7 / 14.9 / 53.7
+// ms, with the refill alone 7.1 / 15.8 / 53.6, packed 3.1 / 19.2 / 49.6, with the
+// stripe terms from powers of z, their bins and marks, and one branch a step
+// 2.3 / 8.8 / 36.8.
+constexpr int kDirectBlock = 8, kDirectRefill = 4, kDirectRound = 32;
+template <int OC>
+constexpr int kDirectBins = OC == kOcStripe ? 2 : 1;
+constexpr int kDirectLongOrbit = 32;
+
+template <int FORM, bool DERIV, int OC>
+struct DirectSample {
+    typename std::conditional<FORM == kFormJulia, JuliaLane<DERIV>, DirectLane<FORM == kFormLane, DERIV>>::type L;
+    typename std::conditional<(OC & kOcTrap) != 0, DirectTrap, char>::type trap;
+    typename std::conditional<OC == kOcStripe && !DERIV, StripeMark, char>::type mark;
+    int entry;
+};
+
+template <int FORM, bool DERIV, int OC>
+__global__ void __launch_bounds__(512) k_direct(DeviceFrame f, ShallowParams p) {
+    using Sample = DirectSample<FORM, DERIV, OC>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_live[16], s_stop;
+    const FrameGeom& g = p.g;
+    const int n_all = f.px.n;
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    const int warps = (int)(blockDim.x >> 5);
+    constexpr int kBins = kDirectBins<OC>;
+    DirectDone* buf = reinterpret_cast<DirectDone*>(smem) + 64 * kBins * warp; // this warp's finished samples
+    Sample* pool = reinterpret_cast<Sample*>(smem + sizeof(DirectDone) * 64 * kBins * warps);
+    Sample S;
+    unsigned long long n_eff = 0, n_steps = 0;
+    unsigned int n_int = 0;
+    int waiting[kBins] = {}, st = kDirectRuns;
+    bool live = false;
+
+    auto run = [&](int steps) {
+#pragma unroll 1
+        for (int k = 0; k < steps && st == kDirectRuns; ++k) {
+            if constexpr (FORM == kFormJulia) {
+                st = S.L.step(p.cr, p.ci, g.mxit, g.ESC2, p.esc_word);
+            } else {
+                st = S.L.step(g.mxit, g.ESC2, p.esc_word, [&](double zr, double zi, double x2, double y2) {
+                    if constexpr ((OC & kOcTrap) != 0) S.trap.push(zr, zi, x2, y2);
+                    if constexpr (OC == kOcStripe && !DERIV) S.mark.visit(S.L.n, zr, zi); // (n: the iterate's index, before it counts)
+                });
+            }
+        }
+    };
+    // takes the warp's ended lanes off and forms 32 values when they are there
+    auto finish = [&]() {
+        __syncwarp();
+        const unsigned ended = __ballot_sync(0xffffffffu, live && st != kDirectRuns);
+        if (ended == 0) return;
+        unsigned in_bin[kBins];
+        if constexpr (kBins == 2) {
+            in_bin[1] = __ballot_sync(0xffffffffu, live && st == kDirectEscaped && S.L.n > kDirectLongOrbit);
+            in_bin[0] = ended & ~in_bin[1];
+        } else {
+            in_bin[0] = ended;
+        }
+        if (live && st != kDirectRuns) {
+            DirectDone d{S.L.x2 + S.L.y2, S.L.dcr, S.L.dci, S.L.zr, S.L.zi, S.L.n, S.entry};
+            if constexpr ((OC & kOcTrap) != 0) {
+                if (!(DERIV && st == kDirectEscaped)) {
+                    d.a = S.trap.point2;
+                    d.b = bitsd(S.trap.cross);
+                    d.zr = S.trap.circle;
+                }
+            }
+            if constexpr (OC == kOcStripe && !DERIV) {
+                d.a = S.mark.zr;
+                d.b = S.mark.zi;
+            }
+            if constexpr (FORM != kFormJulia) {
+                if (st == kDirectOpen) {
+                    DirectEndState e;
+                    OrbitColor<OC & kOcTrap> oc;
+                    st = FORM == kFormLane ? shallow_lane_plain(S.L.cr, S.L.ci, g.mxit, g, e) : shallow_scalar_plain<OC & kOcTrap>(S.L.cr, S.L.ci, g.mxit, g, e, oc);
+                    if (st == kDirectEscaped) d = DirectDone{e.zrad, e.dcr, e.dci, e.zr, e.zi, e.n, S.entry};
+                    if constexpr (OC == kOcStripe && !DERIV) {
+                        if (st == kDirectEscaped && stripe_mark(e.n) > 0) { // the mark, iterated
+                            double zr = S.L.cr, zi = S.L.ci;
+                            for (int k = 0; k < stripe_mark(e.n); ++k) {
+                                const double nzi = d_twice(zr) * zi + S.L.ci;
+                                zr = (zr * zr - zi * zi) + S.L.cr;
+                                zi = nzi;
+                            }
+                            d.a = zr;
+                            d.b = zi;
+                        }
+                    }
+                    if constexpr ((OC & kOcTrap) != 0) {
+                        if (!(DERIV && st == kDirectEscaped)) {
+                            d.a = oc.trap.point2;
+                            d.b = oc.trap.cross;
+                            d.zr = oc.trap.circle;
+                        }
+                    }
+                }
+            }
+            if (st == kDirectInterior) {
+                d.n = -1;
+                n_eff += (unsigned long long)g.mxit;
+                if (FORM == kFormJulia) n_steps += (unsigned long long)g.mxit;
+                ++n_int;
+            } else {
+                n_eff += (unsigned long long)d.n;
+                n_steps += (unsigned long long)d.n;
+            }
+#pragma unroll
+            for (int k = 0; k < kBins; ++k)
+                if ((in_bin[k] >> lane) & 1u) buf[64 * k + waiting[k] + __popc(in_bin[k] & below)] = d;
+            live = false;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < kBins; ++k) {
+            waiting[k] += __popc(in_bin[k]);
+            if (waiting[k] >= 32) {
+                waiting[k] -= 32;
+                direct_write<FORM, OC>(f, p, buf[64 * k + waiting[k] + lane]);
+                __syncwarp();
+            }
+        }
+    };
+
+    for (int rounds = 0;; ++rounds) {
+        const unsigned idle = __ballot_sync(0xffffffffu, !live);
+        const int want = __popc(idle);
+        if (want >= kDirectRefill || (rounds & 3) == 0) {
+            int base = 0;
+            if (lane == 0) {
+                base = n_all;
+                if (!cancelled(f) && (int)*(volatile unsigned int*)&f.ctr->next < n_all) base = want ? (int)atomicAdd(&f.ctr->next, (unsigned)want) : 0;
+            }
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= n_all) break;
+            const int i = base + __popc(idle & below);
+            if (!live && i < n_all) {
+                S.entry = i;
+                int arr[4];
+                entry_key(f.px, i, arr);
+                double cr, ci;
+                direct_c(f, p, arr, cr, ci);
+                if constexpr (FORM == kFormJulia) st = S.L.start(cr, ci, g.ESC2);
+                else st = S.L.start(cr, ci, g.mxit, g.ESC2);
+                if constexpr ((OC & kOcTrap) != 0) S.trap.init();
+                live = true;
+            }
+        }
+        if (live) run(kDirectBlock);
+        finish();
+    }
+    for (;;) {
+        const unsigned m = __ballot_sync(0xffffffffu, live);
+        if (lane == 0) s_live[warp] = __popc(m);
+        if (threadIdx.x == 0) s_stop = cancelled(f) ? 1 : 0;
+        __syncthreads();
+        int total = 0, before = 0, used = 0;
+        for (int w = 0; w < warps; ++w) {
+            const int c = s_live[w];
+            if (w < (int)warp) before += c;
+            total += c;
+            used += c ? 1 : 0;
+        }
+        const bool stop = s_stop != 0;
+        if (total == 0 || stop) break;
+        const bool pack = (total + 31) / 32 < used;
+        if (pack && live) pool[before + __popc(m & below)] = S;
+        __syncthreads();
+        if (pack) {
+            live = (int)threadIdx.x < total;
+            if (live) {
+                S = pool[threadIdx.x];
+                st = kDirectRuns;
+            }
+        }
+        if (live) run(kDirectRound);
+        finish();
+    }
+    // the values still waiting, over the block's warps in full
+#pragma unroll
+    for (int k = 0; k < kBins; ++k) {
+        __syncthreads();
+        if (lane == 0) s_live[warp] = waiting[k];
+        __syncthreads();
+        int t = (int)threadIdx.x, w = 0, total = 0;
+        for (int v = 0; v < warps; ++v) total += s_live[v];
+        for (; t < total; t += (int)blockDim.x) {
+            int at = t;
+            for (w = 0; at >= s_live[w]; ++w) at -= s_live[w];
+            direct_write<FORM, OC>(f, p, reinterpret_cast<DirectDone*>(smem)[64 * (kBins * w + k) + at]);
         }
     }
     atomicAdd(&f.ctr->effective_iters, n_eff);
@@ -1356,23 +1528,41 @@ cudaError_t launch_fe_pass(const DeviceFrame& f, const FeParams& fp, int blocks,
     }
     return cudaGetLastError();
 }
-cudaError_t launch_julia(const DeviceFrame& f, const JuliaParams& jp, int blocks, int threads, cudaStream_t st) {
-    JuliaParams p = jp;
-    p.esc_word = direct_escape_word(p.g.ESC2);
-    k_julia<<<blocks, threads, 0, st>>>(f, p);
+// Blocks of 512 threads, one per SM (four warps a scheduler keep its FP64 unit
+// busy, and the larger the block, the better its last samples pack); frames that
+// would leave SMs without a block take blocks of 128.
+template <int FORM, bool DERIV, int OC>
+static cudaError_t launch_direct(const DeviceFrame& f, const ShallowParams& p, int nsm, cudaStream_t st) {
+    const int threads = f.px.n >= nsm * 512 ? 512 : 128;
+    const int blocks = threads == 512 ? nsm : (f.px.n + 127) / 128;
+    const size_t smem = sizeof(DirectDone) * 2 * kDirectBins<OC> * threads + sizeof(DirectSample<FORM, DERIV, OC>) * threads;
+    auto kern = k_direct<FORM, DERIV, OC>;
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    kern<<<blocks, threads, smem, st>>>(f, p);
     return cudaGetLastError();
 }
-
-cudaError_t launch_shallow(const DeviceFrame& f, const ShallowParams& sp, int blocks, int threads, cudaStream_t st) {
+template <bool DERIV>
+static cudaError_t launch_scalar(const DeviceFrame& f, const ShallowParams& p, int nsm, cudaStream_t st) {
+    switch (p.g.oc) {
+    case 0: return launch_direct<kFormScalar, DERIV, 0>(f, p, nsm, st);
+    case kOcStripe: return launch_direct<kFormScalar, DERIV, kOcStripe>(f, p, nsm, st);
+    default: return launch_direct<kFormScalar, DERIV, kOcTrap>(f, p, nsm, st); // (a trap's value comes before a stripe average's)
+    }
+}
+cudaError_t launch_julia(const DeviceFrame& f, const ShallowParams& jp, int nsm, cudaStream_t st) {
+    ShallowParams p = jp;
+    p.esc_word = direct_escape_word(p.g.ESC2);
+    return p.g.ede ? launch_direct<kFormJulia, true, 0>(f, p, nsm, st) : launch_direct<kFormJulia, false, 0>(f, p, nsm, st);
+}
+cudaError_t launch_shallow(const DeviceFrame& f, const ShallowParams& sp, int nsm, cudaStream_t st) {
     ShallowParams p = sp;
     p.esc_word = direct_escape_word(p.g.ESC2);
-    switch (p.g.oc) {
-    case 0: k_shallow<0><<<blocks, threads, 0, st>>>(f, p); break;
-    case kOcStripe: k_shallow<kOcStripe><<<blocks, threads, 0, st>>>(f, p); break;
-    case kOcTrap: k_shallow<kOcTrap><<<blocks, threads, 0, st>>>(f, p); break;
-    default: k_shallow<kOcStripe | kOcTrap><<<blocks, threads, 0, st>>>(f, p); break;
-    }
-    return cudaGetLastError();
+    if (p.g.oc == 0 && p.simd_semantics) // (no orbit colourings in the lane kernel, mp.cpp:1459)
+        return p.g.ede ? launch_direct<kFormLane, true, 0>(f, p, nsm, st) : launch_direct<kFormLane, false, 0>(f, p, nsm, st);
+    return (p.g.ede || p.g.deovl || p.g.normal) ? launch_scalar<true>(f, p, nsm, st) : launch_scalar<false>(f, p, nsm, st);
 }
 cudaError_t launch_bla_build(const double2* Z, const double2* D, int reflen, double eps, double dcmax, bool ede, double* r2, double4* ab, double4* ce, const int* off, const int* size, int nlev, unsigned long long* rmax2_bits, cudaStream_t st) {
     int n0 = reflen - 1;

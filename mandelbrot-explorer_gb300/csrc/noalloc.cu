@@ -94,8 +94,7 @@ extern "C" int mbx_render_shallow_noalloc(double c0_re, double c0_im, double dx,
     f.cancel = nullptr;
     int dev_sms = 0;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, dev);
-    const int blocks = (int)std::min<size_t>((n + 127) / 128, (size_t)(dev_sms > 0 ? dev_sms * 8 : 1216));
-    if (launch_shallow(f, p, blocks, 128, st) != cudaSuccess) return MBX_E_CUDA;
+    if (launch_shallow(f, p, dev_sms > 0 ? dev_sms : 152, st) != cudaSuccess) return MBX_E_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return MBX_E_CUDA;
     return MBX_OK;
 }

@@ -14,10 +14,11 @@
 // Orbit traps: the orbit's closest approach to the point 0 (|z|), the cross
 // (min(|Re z|, |Im z|), weighted 1.5) and the circle |z| = 1/2; the value is
 // 0.17 (-log10 distance) + 0.025 mu, mu the smooth escape count (0 interior).
-// Operation order follows the reference's, in double; sin, atan2, log and
-// log10 are the platform's (CUDA's on the device).
+// Operation order follows the reference's, in double; the device forms a
+// stripe term by stripe_sin7, and log and log10 are the platform's.
 #pragma once
 #include <math.h>
+#include <string.h>
 
 #ifndef MBX_OC_HD
 #ifdef __CUDACC__
@@ -32,6 +33,49 @@ namespace mbx {
 // coloring bits of the orbit colourings (mbx_request.coloring_method)
 constexpr int kOcStripe = 1, kOcTrap = 2;
 constexpr int kStripeWindow = 256;
+
+MBX_OC_HD unsigned long long oc_bits(double x) {
+#ifdef __CUDA_ARCH__
+    return (unsigned long long)__double_as_longlong(x);
+#else
+    unsigned long long b;
+    memcpy(&b, &x, 8);
+    return b;
+#endif
+}
+MBX_OC_HD double oc_double(unsigned long long b) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)b);
+#else
+    double x;
+    memcpy(&x, &b, 8);
+    return x;
+#endif
+}
+
+// sin(7 arg z) as Im(z^7) / |z|^7: z scaled to [1, 2) by its larger part's binade,
+// four complex products and a reciprocal square root, about 40 FP64 operations
+// where atan2 and sin take over 150. Its error is below theirs (2.5e-15 against
+// 4e-15: theirs begins with the rounding of 7 arg z). For a larger part in
+// [2^-900, 2^900]; the plain form otherwise.
+MBX_OC_HD double stripe_sin7(double zr, double zi) {
+    const double ar = fabs(zr), ai = fabs(zi), m = ar > ai ? ar : ai;
+    if (!(m >= 0x1p-900 && m <= 0x1p900)) return sin(7.0 * atan2(zi, zr));
+    const unsigned long long me = oc_bits(m) >> 52;
+    const double s = oc_double((2046ull - me) << 52); // 2^(1023 - me)
+    const double a = zr * s, b = zi * s;
+    const double aa = a * a, bb = b * b, r2 = aa + bb;
+    const double p2r = aa - bb, p2i = 2.0 * a * b;
+    const double p4r = p2r * p2r - p2i * p2i, p4i = 2.0 * p2r * p2i;
+    const double p6r = p4r * p2r - p4i * p2i, p6i = p4r * p2i + p4i * p2r;
+    const double p7i = p6r * b + p6i * a;
+    const double r4 = r2 * r2, r6 = r4 * r2, r14 = r6 * r6 * r2;
+#ifdef __CUDA_ARCH__
+    return p7i * rsqrt(r14);
+#else
+    return p7i / sqrt(r14);
+#endif
+}
 
 struct StripeAvg {
     double ring[kStripeWindow];
@@ -49,7 +93,11 @@ struct StripeAvg {
         pos = fill = 0;
     }
     MBX_OC_HD void push(double zr, double zi) {
+#ifdef __CUDA_ARCH__
+        const double t = 0.5 + 0.5 * stripe_sin7(zr, zi);
+#else
         const double t = 0.5 + 0.5 * sin(7.0 * atan2(zi, zr));
+#endif
         last = t;
         double out = 0.0;
         if (fill == kStripeWindow) out = ring[pos];
@@ -84,7 +132,7 @@ struct StripeTail {
         fill = 0;
     }
     MBX_OC_HD void push(double zr, double zi) {
-        const double t = 0.5 + 0.5 * sin(7.0 * atan2(zi, zr));
+        const double t = 0.5 + 0.5 * stripe_sin7(zr, zi);
         last = t;
         ++fill;
         tri += (double)kStripeWindow * t - run;
