@@ -59,7 +59,14 @@ MBX_HD df32 operator*(df32 a, df32 b) {
     e = df_fma(a.hi, b.lo, df_fma(a.lo, b.hi, e));
     return df_fast_two_sum(p, e);
 }
-MBX_HD df32 operator/(df32 a, df32 b) {
+// (division and square root are called, not inlined: the lanes that use them are
+// bound by instruction fetch, mixed_lane.cuh)
+#ifdef __CUDACC__
+#define MBX_DF_CALL __host__ __device__ __noinline__ inline
+#else
+#define MBX_DF_CALL inline
+#endif
+MBX_DF_CALL df32 operator/(df32 a, df32 b) {
     const float q1 = a.hi / b.hi;
     const df32 r = a - b * df32(q1);
     const float q2 = (r.hi + r.lo) / b.hi;
@@ -75,7 +82,7 @@ MBX_HD bool operator>=(df32 a, df32 b) { return !(a < b); }
 MBX_HD bool operator==(df32 a, df32 b) { return a.hi == b.hi && a.lo == b.lo; }
 MBX_HD bool operator!=(df32 a, df32 b) { return !(a == b); }
 
-MBX_HD df32 tsqrt(df32 a) {
+MBX_DF_CALL df32 tsqrt(df32 a) {
     if (!(a.hi > 0.0f)) return df32(0.0f);
     const float x = sqrtf(a.hi);
     const df32 r = a - df32(x) * df32(x);

@@ -62,19 +62,24 @@ __device__ __forceinline__ float tlog2(df32 x) { return log2f(x.hi + x.lo); }
 // normal buffer under the DE overlay) or the normal-map angle arg z - arg J;
 // EDE takes precedence, then the normal map. The normal buffer holds 0 where
 // the exact form writes no angle or distance.
+// (once per sample: called, not inlined into the lane kernels)
+__device__ __noinline__ float lane_distance(FE dxfe, double zr2, int sje, double jr, double ji) {
+    const double num = sqrt(zr2) * log(zr2);
+    const FE jmag = fe_mul_d(fe_make(0.5, sje), xsqrt(jr * jr + ji * ji)); // |J| = SJ |(jr, ji)|, SJ = 2^(sje - 1)
+    return (float)fe_to_double(fe_div(fe_from(num), fe_mul(dxfe, jmag)));
+}
+__device__ __noinline__ float lane_normal(double zr, double zi, double jr, double ji) { return (float)(atan2(zi, zr) - atan2(ji, jr)); }
 template <bool DE, class T>
 __device__ __forceinline__ void lane_write_escape(const Outputs& o, const FrameGeom& g, const MixedParams& p, const Lane<T>& L, T zrad) {
     float v = (float)((T)L.iter - tlog2(T(0.5) * tlog2(zrad)));
     if (DE && g.deriv) {
         float nrm = 0.0f;
         if (g.ede || (g.deovl && !g.normal)) {
-            const double zr2 = (double)zrad;
-            const double num = sqrt(zr2) * log(zr2);
-            const float de = (float)fe_to_double(fe_div(fe_from(num), fe_mul(p.dxfe, lane_j_mag(L))));
+            const float de = lane_distance(p.dxfe, (double)zrad, L.SJ.e, (double)L.jr, (double)L.ji);
             if (g.ede) v = de;
             else nrm = de;
         } else if (g.normal) {
-            nrm = (float)(atan2((double)L.ezi, (double)L.ezr) - atan2((double)L.ji, (double)L.jr));
+            nrm = lane_normal((double)L.ezr, (double)L.ezi, (double)L.jr, (double)L.ji);
         }
         if ((g.deovl || g.normal) && o.normal) o.normal[L.oidx] = nrm;
     }

@@ -25,8 +25,14 @@
 
 #ifdef __CUDACC__
 #define MBX_HDF __host__ __device__
+// The lane's rare paths, called: a lane body is tens of kilobytes of
+// instructions, and inlined into it these made the warps wait for instructions
+// more than for anything else (the double-float tier with the derivative was
+// 231 KB; 7.1 warps per issue stalled on instruction fetch).
+#define MBX_RARE __host__ __device__ __noinline__ inline
 #else
 #define MBX_HDF inline
+#define MBX_RARE inline
 #endif
 
 namespace mbx {
@@ -527,12 +533,21 @@ struct Lane {
     T jr, ji, invSJ, ezr, ezi;
 };
 
+// d = dc / S in units of S.
+template <class T>
+MBX_HD typename LaneReal<T>::V2 lane_d(T Sm, int k, typename LaneReal<T>::V2 dcm) {
+    const T inv = fdiv_approx(T(1), Sm);
+    return LaneReal<T>::make2(ldexp_ftz(dcm.x * inv, k), ldexp_ftz(dcm.y * inv, k));
+}
+MBX_RARE df2 lane_d_df(df32 Sm, int k, df2 dcm) { return lane_d<df32>(Sm, k, dcm); }
 template <class T>
 MBX_HD void lane_refresh(Lane<T>& L) {
     L.s = te_to_real(L.S);
-    const T inv = fdiv_approx(T(1), L.S.m);
-    L.dr = ldexp_ftz(L.dcm.x * inv, L.dce - L.S.e);
-    L.di = ldexp_ftz(L.dcm.y * inv, L.dce - L.S.e);
+    typename LaneReal<T>::V2 d;
+    if constexpr (std::is_same<T, df32>::value) d = lane_d_df(L.S.m, L.dce - L.S.e, L.dcm);
+    else d = lane_d<T>(L.S.m, L.dce - L.S.e, L.dcm);
+    L.dr = d.x;
+    L.di = d.y;
 }
 
 // 2^k as a float, |k| <= 126.
@@ -625,48 +640,78 @@ MBX_HD void lane_j_step_2z(Lane<float>& L, float z2r, float z2i) {
     lane_j_window(L);
 }
 
-// J = (nr, ni) given in floatexp.
+// J = (vr, vi) 2^e: SJ takes the binade of the larger part (exact), so SJ.m is
+// always 1/2 and (jr, ji) is J rounded to the lane type once.
 template <class T>
-MBX_HDF void lane_j_set_fe(Lane<T>& L, FE nr, FE ni) {
-    const FE mag = fe_sqrt(fe_add(fe_mul(nr, nr), fe_mul(ni, ni)));
-    if (mag.m == 0.0) {
+MBX_HD void lane_j_set(Lane<T>& L, T vr, T vi, int e) {
+    using R = LaneReal<T>;
+    const typename R::Z ar = tabs(R::z(vr)), ai = tabs(R::z(vi));
+    const typename R::Z amax = ar > ai ? ar : ai;
+    if (!(amax > typename R::Z(0))) { // the derivative vanished (or is not a number)
         L.SJ = TE<T>{T(0.5), 1};
         L.jr = L.ji = T(0);
     } else {
-        L.SJ = te_from_fe<T>(mag);
-        L.jr = (T)fe_to_double(fe_div(nr, mag));
-        L.ji = (T)fe_to_double(fe_div(ni, mag));
+        const int k = te_norm(amax, 0).e; // amax = m 2^k, m in [0.5, 1)
+        L.SJ = TE<T>{T(0.5), e + k + 1};
+        L.jr = lane_mul2k(vr, -k);
+        L.ji = lane_mul2k(vi, -k);
     }
     lane_j_inv(L);
 }
-// J' = 2 z J + 1 with z in floatexp: the steps where z lies outside the lane
-// type's range (the exact floatexp steps; rare).
-template <class T>
-MBX_HDF void lane_j_step_fe(Lane<T>& L, FE zr, FE zi) {
-    const FE sj = fe_from_te(L.SJ);
-    const FE Jr = fe_mul_d(sj, (double)L.jr), Ji = fe_mul_d(sj, (double)L.ji);
+struct JVal { // J = (r, i) 2^e, (r, i) below 1
+    double r, i;
+    int e;
+};
+// J' = 2 z J + 1 with z = X + S w in floatexp: the steps where z lies outside
+// the lane type's range (the exact floatexp steps; rare).
+MBX_RARE JVal lane_j_step_fe(FE Xr, FE Xi, FE S, double wr, double wi, int sje, double jr, double ji) {
+    const FE zr = fe_add(Xr, fe_mul_d(S, wr)), zi = fe_add(Xi, fe_mul_d(S, wi));
+    const FE sj = fe_make(0.5, sje), Jr = fe_mul_d(sj, jr), Ji = fe_mul_d(sj, ji);
     const FE nr = fe_add(fe_scale2(fe_sub(fe_mul(zr, Jr), fe_mul(zi, Ji)), 1), fe_make(0.5, 1));
     const FE ni = fe_scale2(fe_add(fe_mul(zr, Ji), fe_mul(zi, Jr)), 1);
-    lane_j_set_fe(L, nr, ni);
+    const int64_t e = d_is_zero(nr.m) ? ni.e : (d_is_zero(ni.m) ? nr.e : lmax(nr.e, ni.e));
+    return JVal{fe_to_double(fe_make(nr.m, nr.e - e)), fe_to_double(fe_make(ni.m, ni.e - e)), (int)e};
 }
-// J' = A J + B through a BLA skip, with the entry's floatexp coefficients.
+// J' = A J + B through a BLA skip, in pairs of floats for both lane types (the
+// FP32 lane rounds the result to float once; FP64 floatexp, as it was formed
+// before, took some 60 FP64 instructions of 64 cycles a skip and kept the FP32
+// pass's FP64 unit 60 % busy on a 1080p zoom frame).
 template <class T>
-MBX_HDF void lane_j_bla(Lane<T>& L, const BlaEntry<T>& e) {
-    const FE sj = fe_from_te(L.SJ);
-    const FE Jr = fe_mul_d(sj, (double)L.jr), Ji = fe_mul_d(sj, (double)L.ji);
-    const FE Ar = fe_renorm((double)e.ar, e.ea), Ai = fe_renorm((double)e.ai, e.ea);
-    const FE Br = fe_renorm((double)e.br, e.eb), Bi = fe_renorm((double)e.bi, e.eb);
-    const FE nr = fe_add(fe_sub(fe_mul(Ar, Jr), fe_mul(Ai, Ji)), Br);
-    const FE ni = fe_add(fe_add(fe_mul(Ar, Ji), fe_mul(Ai, Jr)), Bi);
-    lane_j_set_fe(L, nr, ni);
-}
-// |J| in floatexp.
+struct JBla {
+    T r, i;
+    int e;
+};
 template <class T>
-MBX_HDF FE lane_j_mag(const Lane<T>& L) {
-    const double jr = (double)L.jr, ji = (double)L.ji;
-    return fe_mul_d(fe_from_te(L.SJ), xsqrt(jr * jr + ji * ji));
+MBX_HD df32 to_df(T x);
+template <>
+MBX_HD df32 to_df<float>(float x) { return df32(x); }
+template <>
+MBX_HD df32 to_df<df32>(df32 x) { return x; }
+template <class T>
+MBX_HD T from_df(df32 x);
+template <>
+MBX_HD float from_df<float>(df32 x) { return x.hi + x.lo; }
+template <>
+MBX_HD df32 from_df<df32>(df32 x) { return x; }
+template <class T>
+MBX_RARE JBla<T> lane_j_bla_df(T Ar, T Ai, int ea, T Br, T Bi, int eb, T Jr, T Ji, int ej) {
+    const df32 ar = to_df(Ar), ai = to_df(Ai), jr = to_df(Jr), ji = to_df(Ji);
+    const df32 tr = ar * jr - ai * ji, ti = ar * ji + ai * jr;
+    const int E1 = ea + ej, E = imax(E1, eb);
+    const df32 vr = ldexp_ftz(tr, E1 - E) + ldexp_ftz(to_df(Br), eb - E);
+    const df32 vi = ldexp_ftz(ti, E1 - E) + ldexp_ftz(to_df(Bi), eb - E);
+    return JBla<T>{from_df<T>(vr), from_df<T>(vi), E};
 }
-
+template <class T>
+MBX_HD void lane_j_bla(Lane<T>& L, const BlaEntry<T>& e) {
+    if constexpr (std::is_same<T, double>::value) {
+        const int E1 = e.ea + L.SJ.e - 1, E = imax(E1, e.eb);
+        lane_j_set(L, ldexp_ftz(e.ar * L.jr - e.ai * L.ji, E1 - E) + ldexp_ftz(e.br, e.eb - E), ldexp_ftz(e.ar * L.ji + e.ai * L.jr, E1 - E) + ldexp_ftz(e.bi, e.eb - E), E);
+    } else {
+        const JBla<T> v = lane_j_bla_df<T>(e.ar, e.ai, e.ea, e.br, e.bi, e.eb, L.jr, L.ji, L.SJ.e - 1);
+        lane_j_set(L, v.r, v.i, v.e);
+    }
+}
 // dz = S w with S <- |v| 2^e and w <- v / |v| for a vector v scaled by 2^e.
 template <class T>
 MBX_HD void lane_set_delta(Lane<T>& L, T vr, T vi, int e) {
@@ -762,12 +807,16 @@ MBX_HD typename LaneReal<T>::E lane_scale_ratio2(TE<T> a, TE<T> b) {
 }
 
 // z = X_m + S w in FP64 (rare decisions).
+MBX_RARE C2 lane_z_fe(double Xr, double Xi, double Sm, int Se, double wr, double wi) {
+    const double sd = xldexp(Sm, Se);
+    return c2(Xr + sd * wr, Xi + sd * wi);
+}
 template <class T>
 MBX_HD void lane_z_double(const Lane<T>& L, const double2* Zd, double& zr, double& zi) {
     const double2 Xd = L.m ? Zd[L.rm] : make_double2(0.0, 0.0);
-    const double sd = xldexp((double)L.S.m, L.S.e);
-    zr = Xd.x + sd * (double)L.wr;
-    zi = Xd.y + sd * (double)L.wi;
+    const C2 z = lane_z_fe(Xd.x, Xd.y, (double)L.S.m, L.S.e, (double)L.wr, (double)L.wi);
+    zr = z.re;
+    zi = z.im;
 }
 
 // The lane's step w' = (2 X + s w) w + d and its error update (one rounding
@@ -859,6 +908,27 @@ MBX_HD void lane_rebase_to(Lane<T>& L, T zr, T zi) {
     L.m = 0;
     L.rm = -1;
     L.Xc = R::make2(T(0), T(0));
+}
+
+// Decision 2 in FP64 floatexp (mp.cpp:3584-3615): z = X + S w against S w, and
+// the new delta (its scale S, 0 when z is, and w).
+struct RebaseFe {
+    bool take;
+    FE S;
+    double wr, wi;
+};
+MBX_RARE RebaseFe lane_rebase_fe(FE S, double wr, double wi, FE Xr, FE Xi, bool force) {
+    const FE Swr = fe_mul_d(S, wr), Swi = fe_mul_d(S, wi);
+    const FE zr = fe_add(Xr, Swr), zi = fe_add(Xi, Swi);
+    const FE zrad = fe_add(fe_mul(zr, zr), fe_mul(zi, zi));
+    const FE dz = fe_add(fe_mul(Swr, Swr), fe_mul(Swi, Swi));
+    RebaseFe v{force || fe_abs_less(zrad, dz), fe_make(0.0, 0), 0.0, 0.0};
+    if (!v.take) return v;
+    v.S = fe_sqrt(zrad);
+    if (v.S.m == 0.0) return v;
+    v.wr = fe_to_double(fe_div(zr, v.S));
+    v.wi = fe_to_double(fe_div(zi, v.S));
+    return v;
 }
 
 // Common iterations of the FP32 lane without interior detection. The
@@ -1322,8 +1392,8 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                 lane_j_advance(L);
             } else { // z outside the lane type's range: in floatexp
                 const FE zero = fe_make(0.0, 0);
-                const FE S0 = fe_from_te(L.S);
-                lane_j_step_fe(L, fe_add(L.m ? Zfe[L.rm].re : zero, fe_mul_d(S0, (double)L.wr)), fe_add(L.m ? Zfe[L.rm].im : zero, fe_mul_d(S0, (double)L.wi)));
+                const JVal v = lane_j_step_fe(L.m ? Zfe[L.rm].re : zero, L.m ? Zfe[L.rm].im : zero, fe_from_te(L.S), (double)L.wr, (double)L.wi, L.SJ.e, (double)L.jr, (double)L.ji);
+                lane_j_set(L, (T)v.r, (T)v.i, v.e);
             }
         }
         if (!tiny) {
@@ -1547,21 +1617,15 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
             }
         } else if (decide == 2) {
             ++n_ferebase;
-            const FE S = fe_from_te(L.S);
-            FE Xmr = L.m ? Zfe[L.rm].re : fe_make(0.0, 0);
-            FE Xmi = L.m ? Zfe[L.rm].im : fe_make(0.0, 0);
-            FE Swr = fe_mul_d(S, (double)L.wr), Swi = fe_mul_d(S, (double)L.wi);
-            FE zrfe = fe_add(Xmr, Swr), zife = fe_add(Xmi, Swi);
-            FE zradfe = fe_add(fe_mul(zrfe, zrfe), fe_mul(zife, zife));
-            FE dzfe = fe_add(fe_mul(Swr, Swr), fe_mul(Swi, Swi));
-            if ((!per && L.m >= reflen) || fe_abs_less(zradfe, dzfe)) {
-                FE Snew = fe_sqrt(zradfe);
-                if (Snew.m == 0.0) {
+            const FE zero = fe_make(0.0, 0);
+            const RebaseFe v = lane_rebase_fe(fe_from_te(L.S), (double)L.wr, (double)L.wi, L.m ? Zfe[L.rm].re : zero, L.m ? Zfe[L.rm].im : zero, !per && L.m >= reflen);
+            if (v.take) {
+                if (v.S.m == 0.0) {
                     L.wr = L.wi = T(0);
                 } else {
-                    L.S = te_from_fe<T>(Snew);
-                    L.wr = (T)fe_to_double(fe_div(zrfe, Snew));
-                    L.wi = (T)fe_to_double(fe_div(zife, Snew));
+                    L.S = te_from_fe<T>(v.S);
+                    L.wr = (T)v.wr;
+                    L.wi = (T)v.wi;
                     lane_refresh(L);
                     if (R::kTrackError) L.err2 = L.err2 * lane_scale_ratio2(S0, L.S) + R::kEps2;
                 }
