@@ -225,7 +225,7 @@ class Engine {
     DevBuf<float2> dZf_;
     DevBuf<float4> dZq_;  // FP32 lane's common-step orbit table (MixedParams::Zq)
     DevBuf<Bla32> dbla32_;
-    DevBuf<BlaMaxR2> dblamax_;
+    DevBuf<BlaMaxR2> dblamax_, dblamaxdf_;
     bool blamax_ok_ = false; // dblamax_ holds the current reference's table
     DevBuf<BlaDF> dbladf_;
     DevBuf<df2> dZdf_;

@@ -45,9 +45,9 @@ struct __align__(16) BlaEntry {
 using Bla32 = BlaEntry<float>;
 using BlaDF = BlaEntry<df32>;
 using Bla64 = BlaEntry<double>;
-// Per BLA position of the FP32 lane (orbit index s with s - 1 a multiple of
+// Per BLA position of a lane (orbit index s with s - 1 a multiple of
 // 2^minlevel): the largest radius^2 over the levels the lane tries there, as
-// mantissa + exponent of the FP32 table; m = 0 when no level has a radius. A
+// mantissa (its high part) + exponent of the lane's table; m = 0 when no level has a radius. A
 // |dz|^2 at or above it fails every level's radius test.
 struct BlaMaxR2 {
     float m;
@@ -246,6 +246,7 @@ struct MixedParams {
     const float* dpx_tabf = nullptr;
     const float* dpy_tabf = nullptr;
     const BlaMaxR2* blamax = nullptr; // FP32 lane: index (s - 1) >> minlevel
+    const BlaMaxR2* blamax_df = nullptr; // double-float lane, the same from its table
     int probe_stop = 0;               // interior gate probe: stop at the first interior decision
     unsigned wide_from = 0;  // rerun passes launched in two widths: the 32-lane
                              // variant runs when the queue holds >= wide_from

@@ -32,9 +32,10 @@ __global__ void k_bla_to_lane(const double* r2, const double4* ab, BlaEntry<T>* 
     if (i < n) out[i] = bla_entry<T>(r2[i], ab[i]);
 }
 
-// The FP32 lane's per-position radius maxima (BlaMaxR2): the levels lane_bla
+// The lanes' per-position radius maxima (BlaMaxR2): the levels lane_bla
 // tries at s, startp down to minlevel, as it orders them.
-__global__ void k_bla_maxr2(const BlaEntry<float>* t, BlaView b, BlaMaxR2* out, int nq) {
+template <class T>
+__global__ void k_bla_maxr2(const BlaEntry<T>* t, BlaView b, BlaMaxR2* out, int nq) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nq) return;
     const int s = (q << b.minlevel) + 1;
@@ -45,9 +46,11 @@ __global__ void k_bla_maxr2(const BlaEntry<float>* t, BlaView b, BlaMaxR2* out, 
     for (int p = startp; p >= b.minlevel; --p) {
         const int i = (s - 1) >> p;
         if (i >= b.size[p]) continue;
-        const BlaEntry<float> e = t[b.off[p] + i];
-        if (e.r2m == 0.0f) continue;
-        if (best.m == 0.0f || e.r2e > best.e || (e.r2e == best.e && e.r2m > best.m)) best = BlaMaxR2{e.r2m, e.r2e};
+        const BlaEntry<T>& e = t[b.off[p] + i];
+        const float r2m = LaneReal<T>::z(e.r2m);
+        const int r2e = e.r2e;
+        if (r2m == 0.0f) continue;
+        if (best.m == 0.0f || r2e > best.e || (r2e == best.e && r2m > best.m)) best = BlaMaxR2{r2m, r2e};
     }
     out[q] = best;
 }
@@ -525,9 +528,10 @@ int Engine::prepare_mixed() {
         k_bla_to_lane<float><<<(n + 255) / 256, 256, 0, st_>>>(dr2_.p, dab_.p, dbla32_.p, n);
         k_bla_to_lane<df32><<<(n + 255) / 256, 256, 0, st_>>>(dr2_.p, dab_.p, dbladf_.p, n);
         const int nq = (len >> bla_.minlevel) + 2;
-        if (!ensure(dblamax_, (size_t)nq)) return MBX_E_NOMEM;
-        k_bla_maxr2<<<(nq + 255) / 256, 256, 0, st_>>>(dbla32_.p, bla_, dblamax_.p, nq);
-        stats_.kernel_launches += 3;
+        if (!ensure(dblamax_, (size_t)nq) || !ensure(dblamaxdf_, (size_t)nq)) return MBX_E_NOMEM;
+        k_bla_maxr2<float><<<(nq + 255) / 256, 256, 0, st_>>>(dbla32_.p, bla_, dblamax_.p, nq);
+        k_bla_maxr2<df32><<<(nq + 255) / 256, 256, 0, st_>>>(dbladf_.p, bla_, dblamaxdf_.p, nq);
+        stats_.kernel_launches += 4;
         blamax_ok_ = true;
     } else {
         blamax_ok_ = false;
@@ -557,6 +561,7 @@ MixedParams Engine::mixed_params() const {
     p.wmax2 = mixed_wmax2_;
     p.wmin2 = 1.0f / mixed_wmax2_;
     p.blamax = blamax_ok_ ? dblamax_.p : nullptr;
+    p.blamax_df = blamax_ok_ ? dblamaxdf_.p : nullptr;
     if (ddpxy_.p && dpxy_w_ == W_ * SUB_) {
         p.dpx_tab = ddpxy_.p;
         p.dpy_tab = ddpxy_.p + dpxy_w_;

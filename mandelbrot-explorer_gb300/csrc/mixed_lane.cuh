@@ -533,6 +533,11 @@ struct Lane {
     T jr, ji, invSJ, ezr, ezi;
 };
 
+// 2 x, exactly (of a double-float: both parts; what the product with 2 gives)
+MBX_HD float lane_twice(float x) { return x + x; }
+MBX_HD double lane_twice(double x) { return x + x; }
+MBX_HD df32 lane_twice(df32 x) { return df32(x.hi + x.hi, x.lo + x.lo); }
+
 // d = dc / S in units of S.
 template <class T>
 MBX_HD typename LaneReal<T>::V2 lane_d(T Sm, int k, typename LaneReal<T>::V2 dcm) {
@@ -625,8 +630,8 @@ MBX_HD void lane_j_window(Lane<T>& L) {
 // J' = 2 z J + 1 with z at unit scale in the lane type.
 template <class T>
 MBX_HD void lane_j_step(Lane<T>& L, T zr, T zi) {
-    const T a = T(2) * (zr * L.jr - zi * L.ji) + L.invSJ;
-    const T b = T(2) * (zr * L.ji + zi * L.jr);
+    const T a = lane_twice(zr * L.jr - zi * L.ji) + L.invSJ;
+    const T b = lane_twice(zr * L.ji + zi * L.jr);
     L.jr = a;
     L.ji = b;
     lane_j_window(L);
@@ -825,8 +830,8 @@ template <class T>
 MBX_HD void lane_step(typename LaneReal<T>::V2 X, T s, T wr, T wi, T dr, T di, typename LaneReal<T>::E err2, typename LaneReal<T>::E g2, T& nwr, T& nwi,
                       typename LaneReal<T>::E& nerr2) {
     using R = LaneReal<T>;
-    const T fR = T(2) * X.x + s * wr;
-    const T fI = T(2) * X.y + s * wi;
+    const T fR = lane_twice(X.x) + s * wr;
+    const T fI = lane_twice(X.y) + s * wi;
     nwr = fR * wr - fI * wi + dr;
     nwi = fR * wi + fI * wr + di;
     const typename R::E a = R::toe(nwr), c = R::toe(nwi);
@@ -1271,7 +1276,7 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
             if (!intr || FASTI) {
                 using E = typename R::E;
                 const Z wmax2 = Z(p.wmax2), wmin2 = Z(p.wmin2);
-                const BlaMaxR2* bmax = std::is_same<T, float>::value ? p.blamax : nullptr; // FP32 tables only
+                const BlaMaxR2* bmax = std::is_same<T, float>::value ? p.blamax : p.blamax_df;
                 const int minlevel = f.bla.minlevel;
                 // one counter: m; iter = m + off, the steps taken and the
                 // budget spent follow from m - m0 and are written back on exit.
@@ -1287,6 +1292,16 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                 // general code would not rebase
                 const Z s2x5 = Z(5.0001) * (R::z(L.s) * R::z(L.s));
                 int m = m0;
+                // the double-float lane carries s w: z = X + s w now and
+                // f = 2 X + s w of the next step take the same product, and J's
+                // pre-step z is the z of the step before
+                T tr = T(0), ti = T(0), zpr = T(0), zpi = T(0);
+                if constexpr (!std::is_same<T, float>::value) {
+                    tr = L.s * L.wr;
+                    ti = L.s * L.wi;
+                    zpr = L.Xc.x + tr;
+                    zpi = L.Xc.y + ti;
+                }
                 for (;;) {
                     if (m >= mlim) break;
                     if (FASTI && intr) {
@@ -1311,8 +1326,22 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                     const typename R::V2 X = orb[nrm];
                     T nwr, nwi;
                     E nerr2;
-                    lane_step<T>(L.Xc, L.s, L.wr, L.wi, L.dr, L.di, L.err2, L.g2, nwr, nwi, nerr2);
-                    const T zr = lane_zc<T>(X.x, L.s, nwr), zi = lane_zc<T>(X.y, L.s, nwi);
+                    T zr, zi, ntr, nti;
+                    if constexpr (std::is_same<T, float>::value) {
+                        lane_step<T>(L.Xc, L.s, L.wr, L.wi, L.dr, L.di, L.err2, L.g2, nwr, nwi, nerr2);
+                        zr = lane_zc<T>(X.x, L.s, nwr);
+                        zi = lane_zc<T>(X.y, L.s, nwi);
+                    } else { // lane_step and lane_zc
+                        const T fR = lane_twice(L.Xc.x) + tr, fI = lane_twice(L.Xc.y) + ti;
+                        nwr = fR * L.wr - fI * L.wi + L.dr;
+                        nwi = fR * L.wi + fI * L.wr + L.di;
+                        const E a = R::toe(nwr), c = R::toe(nwi);
+                        nerr2 = L.err2 * L.g2 + R::kEps2 * (a * a + c * c);
+                        ntr = L.s * nwr;
+                        nti = L.s * nwi;
+                        zr = X.x + ntr;
+                        zi = X.y + nti;
+                    }
                     const Z zrad = R::zabs2(zr, zi);
                     const Z wm2 = R::zabs2(nwr, nwi);
                     const Z xr2 = R::zabs2(X.x, X.y);
@@ -1321,7 +1350,17 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                     // |w|^2 tests: the general code handles them)
                     const bool rare = zrad > ESC2lo || !(nerr2 <= kLaneCap2 * (E)wm2) || wm2 > wmax2 || wm2 < wmin2 || !far;
                     if (rare) break;
-                    if (deriv) lane_j_advance(L); // (from the pre-step state)
+                    if constexpr (std::is_same<T, float>::value) {
+                        if (deriv) lane_j_advance(L); // (from the pre-step state)
+                    } else {
+                        if (deriv) {
+                            lane_j_step(L, zpr, zpi);
+                            zpr = zr;
+                            zpi = zi;
+                        }
+                        tr = ntr;
+                        ti = nti;
+                    }
                     L.wr = nwr;
                     L.wi = nwi;
                     L.err2 = nerr2;
