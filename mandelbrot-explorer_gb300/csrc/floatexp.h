@@ -71,26 +71,40 @@ MBX_HD double d_twice(double x) {
     return x; // infinity, NaN
 }
 
+// The floatexp operations run in the exact loop's serial chains, where an integer
+// instruction costs its latency like an FP64 one (a BLA skip took some 750 of them
+// beside 75 FP64 ones): each has one test for its common case (normal mantissas,
+// in-range results) and leaves the others to a called function.
+#ifdef __CUDACC__
+#define MBX_COLD __host__ __device__ __noinline__ inline
+#else
+#define MBX_COLD inline
+#endif
+
 // frexp: x = r * 2^e with 0.5 <= |r| < 1; zero, inf and nan return x with e = 0.
-MBX_HD double xfrexp(double x, int* e) {
+struct FrexpOf {
+    double m;
+    int e;
+};
+MBX_COLD FrexpOf xfrexp_rare(double x) { // zero, subnormal, infinite, NaN
     uint64_t b = dbits(x);
     int ex = (int)((b >> 52) & 0x7ff);
-    int adj = 0;
-    if (ex == 0) {
-        if ((b << 1) == 0) {
-            *e = 0;
-            return x;
-        }
-        x = x * 18014398509481984.0; // 2^54, exact
-        b = dbits(x);
-        ex = (int)((b >> 52) & 0x7ff);
-        adj = -54;
-    } else if (ex == 0x7ff) {
-        *e = 0;
-        return x;
+    if (ex != 0 || (b << 1) == 0) return FrexpOf{x, 0};
+    x = x * 18014398509481984.0; // 2^54, exact
+    b = dbits(x);
+    ex = (int)((b >> 52) & 0x7ff);
+    return FrexpOf{bitsd((b & 0x800fffffffffffffull) | (1022ull << 52)), ex - 1022 - 54};
+}
+MBX_HD bool d_normal(uint64_t b) { return (unsigned)((b >> 52) & 0x7ff) - 1u < 0x7feu; }
+MBX_HD double xfrexp(double x, int* e) {
+    const uint64_t b = dbits(x);
+    if (d_normal(b)) {
+        *e = (int)((b >> 52) & 0x7ff) - 1022;
+        return bitsd((b & 0x800fffffffffffffull) | (1022ull << 52));
     }
-    *e = ex - 1022 + adj;
-    return bitsd((b & 0x800fffffffffffffull) | (1022ull << 52));
+    const FrexpOf r = xfrexp_rare(x);
+    *e = r.e;
+    return r.m;
 }
 
 // Exact power of two 2^k for -1074 <= k <= 1023 (subnormal below -1022).
@@ -100,7 +114,7 @@ MBX_HD double pow2i(int k) {
 }
 
 // ldexp for finite x, correctly rounded (one rounding in the subnormal range).
-MBX_HD double xldexp(double x, int k) {
+MBX_COLD double xldexp_rare(double x, int k) {
     if (d_is_zero(x)) return x;
     uint64_t b = dbits(x);
     if (((b >> 52) & 0x7ff) == 0x7ff) return x;
@@ -116,35 +130,44 @@ MBX_HD double xldexp(double x, int k) {
     // 2^ne is exactly representable here; one multiply gives the one rounding.
     return m * pow2i((int)ne);
 }
+MBX_HD double xldexp(double x, int k) {
+    const uint64_t b = dbits(x);
+    // normal x, normal result: the exponent field moves
+    if (d_normal(b) && (unsigned)((b >> 52) & 0x7ff) - 1u + (unsigned)k < 0x7feu) return bitsd(b + ((uint64_t)(int64_t)k << 52));
+    return xldexp_rare(x, k);
+}
 
+// m 2^e; the exponent is an int (|e| stays far below 2^31: a scale of 10^k needs
+// k decimal digits).
 struct FE {
     double m;
-    int64_t e;
+    int e;
 };
 
-MBX_HD FE fe_make(double m, int64_t e) {
+MBX_HD FE fe_make(double m, int e) {
     FE r;
     r.m = m;
     r.e = e;
     return r;
 }
-MBX_HD FE fe_from(double x) {
-    if (d_is_zero(x)) return fe_make(0.0, 0);
-    int ex;
-    double mm = xfrexp(x, &ex);
-    return fe_make(mm, (int64_t)ex);
+MBX_HD FE fe_renorm(double m, int e) {
+    const uint64_t b = dbits(m);
+    if (d_normal(b)) return fe_make(bitsd((b & 0x800fffffffffffffull) | (1022ull << 52)), e + (int)((b >> 52) & 0x7ff) - 1022);
+    if (d_is_zero(m)) return fe_make(0.0, 0);
+    const FrexpOf r = xfrexp_rare(m);
+    return fe_make(r.m, e + r.e);
+}
+MBX_HD FE fe_from(double x) { return fe_renorm(x, 0); }
+MBX_COLD double fe_to_double_rare(FE a) {
+    if (d_is_zero(a.m)) return 0.0;
+    if (a.e > 1100) return bitsd(0x7ff0000000000000ull | (dbits(a.m) & 0x8000000000000000ull));
+    if (a.e < -1100) return 0.0;
+    return xldexp(a.m, a.e);
 }
 MBX_HD double fe_to_double(FE a) {
-    if (d_is_zero(a.m)) return 0.0;
-    if (a.e > 1100) return bitsd(a.m > 0 ? 0x7ff0000000000000ull : 0xfff0000000000000ull);
-    if (a.e < -1100) return 0.0;
-    return xldexp(a.m, (int)a.e);
-}
-MBX_HD FE fe_renorm(double m, int64_t e) {
-    if (d_is_zero(m)) return fe_make(0.0, 0);
-    int ex;
-    double mm = xfrexp(m, &ex);
-    return fe_make(mm, e + ex);
+    const uint64_t b = dbits(a.m);
+    if (d_normal(b) && (unsigned)((b >> 52) & 0x7ff) - 1u + (unsigned)a.e < 0x7feu) return bitsd(b + ((uint64_t)(int64_t)a.e << 52));
+    return fe_to_double_rare(a);
 }
 MBX_HD FE fe_mul(FE a, FE b) {
     if (d_is_zero(a.m) || d_is_zero(b.m)) return fe_make(0.0, 0);
@@ -154,15 +177,17 @@ MBX_HD FE fe_mul_d(FE a, double b) {
     if (d_is_zero(a.m) || d_is_zero(b)) return fe_make(0.0, 0);
     return fe_renorm(a.m * b, a.e);
 }
-MBX_HD FE fe_scale2(FE a, int64_t k) { return d_is_zero(a.m) ? a : fe_make(a.m, a.e + k); }
+MBX_HD FE fe_scale2(FE a, int k) { return d_is_zero(a.m) ? a : fe_make(a.m, a.e + k); }
 MBX_HD FE fe_add(FE a, FE b) {
     if (d_is_zero(a.m)) return b;
     if (d_is_zero(b.m)) return a;
-    int64_t d = a.e - b.e;
+    const int d = a.e - b.e;
     if (d > 54) return a;
     if (d < -54) return b;
-    if (d >= 0) return fe_renorm(a.m + xldexp(b.m, -(int)d), a.e);
-    return fe_renorm(b.m + xldexp(a.m, (int)d), b.e);
+    // the smaller exponent's mantissa aligned to the larger (one add for both orders)
+    const bool first = d >= 0;
+    const double big = first ? a.m : b.m, small = xldexp(first ? b.m : a.m, first ? -d : d);
+    return fe_renorm(big + small, first ? a.e : b.e);
 }
 MBX_HD FE fe_neg(FE a) { return fe_make(-a.m, a.e); }
 MBX_HD FE fe_sub(FE a, FE b) { return fe_add(a, fe_neg(b)); }
@@ -184,11 +209,11 @@ MBX_HD double xsqrt(double x) {
 #endif
 }
 MBX_HD FE fe_sqrt(FE a) {
-    if (a.m <= 0.0) return fe_make(0.0, 0);
-    int64_t e = a.e;
+    if (d_le_zero(a.m)) return fe_make(0.0, 0);
+    int e = a.e;
     double m = a.m;
     if (e & 1) {
-        m *= 2.0;
+        m = d_twice(m);
         --e;
     }
     return fe_renorm(xsqrt(m), e / 2);

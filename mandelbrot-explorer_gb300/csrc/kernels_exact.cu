@@ -337,9 +337,9 @@ __device__ void bla_rerescale_underflow(FE& S, double& wr, double& wi, double nw
 
 __device__ void fe_step_underflow(FE Xr, FE Xi, FE dcr, FE dci, FE& S, double& wr, double& wi) { // mp.cpp:2794-2835
     const double sm = S.m, sm2 = sm * sm;
-    const int64_t se = S.e;
-    const int64_t NONE = (int64_t)0x8000000000000000ll;
-    int64_t e = NONE;
+    const int se = S.e;
+    const int NONE = (int)0x80000000;
+    int e = NONE;
     const bool has_w = wr != 0.0 || wi != 0.0;
     if (has_w && Xr.m != 0.0) e = max(e, Xr.e + se);
     if (has_w && Xi.m != 0.0) e = max(e, Xi.e + se);
@@ -351,10 +351,10 @@ __device__ void fe_step_underflow(FE Xr, FE Xi, FE dcr, FE dci, FE& S, double& w
         wr = wi = 0.0;
         return;
     }
-    auto align = [e](double m, int64_t te) -> double {
-        int64_t d = te - e;
+    auto align = [e](double m, int te) -> double {
+        int d = te - e;
         if (m == 0.0 || d < -54) return 0.0;
-        return m * pow2i((int)d);
+        return m * pow2i(d);
     };
     const double xs_r = align(Xr.m * sm, Xr.e + se);
     const double xs_i = align(Xi.m * sm, Xi.e + se);
@@ -377,20 +377,20 @@ __device__ void fe_step_underflow(FE Xr, FE Xi, FE dcr, FE dci, FE& S, double& w
 
 __device__ void fe_deriv_underflow(FE zr, FE zi, FE& SJ, double& jr, double& ji, double& invSJd) { // mp.cpp:2842-2876
     double im = 0.5 / SJ.m;
-    int64_t ie = 1 - SJ.e;
+    int ie = 1 - SJ.e;
     if (im >= 1.0) {
         im *= 0.5;
         ++ie;
     }
     FE invSJ = fe_make(im, ie);
-    int64_t e = invSJ.e;
+    int e = invSJ.e;
     if (zr.m != 0.0) e = max(e, zr.e);
     if (zi.m != 0.0) e = max(e, zi.e);
     auto align = [e](FE x) -> double {
         if (x.m == 0.0) return 0.0;
-        int64_t d = x.e - e;
+        int d = x.e - e;
         if (d < -54) return 0.0;
-        return x.m * pow2i((int)d);
+        return x.m * pow2i(d);
     };
     double azr = align(zr), azi = align(zi);
     double ar = 2.0 * (azr * jr - azi * ji) + align(invSJ);
@@ -421,7 +421,7 @@ __device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int
         // |w|^2 >= (the larger part)^2 >= 2^(2 k), k its binade, so |dz|^2's
         // exponent is at least S2.e + 2 k: above rmax2's, no radius holds
         const unsigned h = umax_(hi_abs(wr), hi_abs(wi));
-        const int64_t lo = S2.e + 2 * ((int64_t)(h >> 20) - 1023);
+        const int lo = S2.e + 2 * ((int)(h >> 20) - 1023);
         if (h >= 0x20000000u && h < 0x5fe00000u && !d_is_zero(S2.m) && lo > rmax.e) return 0;
     }
     const FE dz2 = fe_mul(S2, fe_from(wr * wr + wi * wi));
@@ -429,8 +429,13 @@ __device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int
     for (int p = startp; p >= b.minlevel; --p) {
         int i = (s - 1) >> p;
         if (i >= b.size[p]) continue;
-        double r2 = b.r2[b.off[p] + i];
-        if (d_le_zero(r2) || !fe_abs_less(dz2, fe_from(r2))) continue;
+        const double r2 = b.r2[b.off[p] + i];
+        // |dz|^2 < r2, on exponents and mantissa bits (r2 normal) or in floatexp
+        const uint64_t rb = dbits(r2);
+        const int re = (int)(rb >> 52) - 1022;
+        if ((int64_t)rb > 0 && d_normal(rb) ? !(dz2.e < re || (dz2.e == re && (dbits(dz2.m) & 0xfffffffffffffull) < (rb & 0xfffffffffffffull))) && !d_is_zero(dz2.m)
+                                            : d_le_zero(r2) || !fe_abs_less(dz2, fe_from(r2)))
+            continue;
         int l = 1 << p;
         int land = s + l;
         if (land >= mx_ref_it - 1) continue;
@@ -443,7 +448,7 @@ __device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int
             // z = Z_land + S n: with each part of Z_land and of S n below 4, |z|^2
             // is below 128, so only a bailout^2 below that needs z itself
             const unsigned hn = umax_(hi_abs(nwr), hi_abs(nwi));
-            if (!(umax_(hi_abs(zl.x), hi_abs(zl.y)) < 0x40100000u && (int64_t)(hn >> 20) - 1022 + S.e <= 2 && d_abs_less(200.0, ESC2))) {
+            if (!(umax_(hi_abs(zl.x), hi_abs(zl.y)) < 0x40100000u && (int)(hn >> 20) - 1022 + S.e <= 2 && d_abs_less(200.0, ESC2))) {
                 double fr = zl.x + fe_to_double(fe_mul_d(S, nwr));
                 double fi = zl.y + fe_to_double(fe_mul_d(S, nwi));
                 if (d_abs_less(ESC2, fr * fr + fi * fi)) return 0; // > ESC2
@@ -533,7 +538,7 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
     int rm = 0;
     FE S = fe_sqrt(fe_add(fe_mul(dcr, dcr), fe_mul(dci, dci)));
     double wr, wi, dr, di;
-    if (S.m == 0.0) {
+    if (d_is_zero(S.m)) {
         S = fe_make(1.0, 0);
         wr = wi = dr = di = 0.0;
     } else {
@@ -596,7 +601,7 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
                     FE nJr = fe_add(fe_sub(fe_mul_d(Jr, ab[0]), fe_mul_d(Ji, ab[1])), fe_from(ab[2]));
                     FE nJi = fe_add(fe_add(fe_mul_d(Jr, ab[1]), fe_mul_d(Ji, ab[0])), fe_from(ab[3]));
                     SJ = fe_sqrt(fe_add(fe_mul(nJr, nJr), fe_mul(nJi, nJi)));
-                    if (SJ.m == 0.0) {
+                    if (d_is_zero(SJ.m)) {
                         SJ = fe_make(1.0, 0);
                         jr = ji = 0.0;
                         invSJd = 1.0;
@@ -792,7 +797,7 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
             FE dzfe = fe_add(fe_mul(Swr, Swr), fe_mul(Swi, Swi));
             if ((!per && m >= reflen) || fe_abs_less(zradfe, dzfe)) {
                 FE Snew = fe_sqrt(zradfe);
-                if (Snew.m == 0.0) {
+                if (d_is_zero(Snew.m)) {
                     wr = wi = 0.0;
                 } else {
                     S = Snew;
