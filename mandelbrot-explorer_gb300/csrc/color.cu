@@ -10,8 +10,10 @@
 // logf/powf are correctly rounded on all but ~1e-4 of inputs); tables built on
 // the host with the host's libm for the functions of the palette entry
 // (powf(c/255, 2.2)) and of the final byte (a monotone step function of the
-// linear value, stored as its 352 step positions); the FP64 library tanh, cos,
-// sin and sqrt for the distance mapping and the two shadings.
+// linear value, stored as its 352 step positions); the relief shade and the
+// shaded sums in pairs of floats where those settle their rounding to float
+// (color_math.cuh), else in double; the FP64 library tanh, cos, sin and sqrt for
+// the distance mapping and the normal map.
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -115,13 +117,14 @@ namespace {
 // and NaN give INT_MIN (render.cpp:89 on values past 2^31 / 2048).
 __device__ __forceinline__ int trunc_i32(float y) { return fabsf(y) < 2147483648.0f ? (int)y : (int)0x80000000u; }
 
+__device__ __noinline__ float tanh_fp64(float t) { return __double2float_rn(tanh((double)t)); }
 __device__ __forceinline__ int palette_index(float v, int mapping, float density, const cm::Exp2Table& tab, int& fb) {
     float f;
     if (mapping == MBX_MAP_STRIPE) {
         f = cm::mul(v, cm::div(density, 20.0f));
     } else if (mapping == MBX_MAP_DISTANCE) {
         const float t = cm::mul(cm::div(cm::mul(v, density), 3600.0f), 5.0f);
-        f = __double2float_rn(tanh((double)t));
+        f = tanh_fp64(t);
     } else if (mapping == MBX_MAP_TRAP) {
         f = v;
     } else {
@@ -136,8 +139,17 @@ __device__ __forceinline__ int palette_index(float v, int mapping, float density
     return i;
 }
 
-// render.cpp:47-69 on the supersampled grid.
-__device__ float relief_shade(const float* __restrict__ v, int y, int x, int ws, int hs, double strength, double lx, double ly, double lz) {
+// render.cpp:47-69 on the supersampled grid: in pairs of floats, or in double
+// where those leave the rounding to float open.
+__device__ __noinline__ float relief_double(float sx, float sy, double strength, double lx, double ly, double lz) {
+    const double nx = __dmul_rn((double)(-sx), strength), ny = __dmul_rn((double)(-sy), strength);
+    const double inv = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, nx), __dmul_rn(ny, ny)), 1.0)));
+    double d = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, lx), __dmul_rn(ny, ly)), lz), inv);
+    if (d < 0) d = 0;
+    return __double2float_rn(__dadd_rn(0.25, __dmul_rn(0.85, d)));
+}
+__device__ __forceinline__ float relief_shade(const ColorLaunch& a, int y, int x, int ws, int hs) {
+    const float* __restrict__ v = a.values;
     const float c = v[(size_t)y * ws + x];
     if (c < 0) return 1.0f;
     auto at = [&](int yy, int xx) -> float {
@@ -147,15 +159,13 @@ __device__ float relief_shade(const float* __restrict__ v, int y, int x, int ws,
     };
     const float sx = cm::mul(cm::sub(at(y, x + 1), at(y, x - 1)), 0.5f);
     const float sy = cm::mul(cm::sub(at(y + 1, x), at(y - 1, x)), 0.5f);
-    const double nx = __dmul_rn((double)(-sx), strength), ny = __dmul_rn((double)(-sy), strength);
-    const double inv = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, nx), __dmul_rn(ny, ny)), 1.0)));
-    double d = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, lx), __dmul_rn(ny, ly)), lz), inv);
-    if (d < 0) d = 0;
-    return __double2float_rn(__dadd_rn(0.25, __dmul_rn(0.85, d)));
+    float out;
+    if (cm::relief_ff(sx, sy, a.relief_ff, out)) return out;
+    return relief_double(sx, sy, a.relief, a.lx, a.ly, a.lz);
 }
 
 // render.cpp:276-287.
-__device__ float normal_shade(float ang, double lx, double ly, double lz) {
+__device__ __noinline__ float normal_shade(float ang, double lx, double ly, double lz) {
     const double nx = cos((double)ang), ny = sin((double)ang);
     const double inv = __ddiv_rn(1.0, __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, nx), __dmul_rn(ny, ny)), 1.0)));
     double d = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(nx, lx), __dmul_rn(ny, ly)), lz), inv);
@@ -163,8 +173,10 @@ __device__ float normal_shade(float ang, double lx, double ly, double lz) {
     return __double2float_rn(__dadd_rn(0.3, __dmul_rn(0.8, d)));
 }
 
+__device__ __noinline__ float acc_shaded_double(float acc, float c, float sh) { return __double2float_rn(__dadd_rn((double)acc, __dmul_rn((double)c, (double)sh))); }
 __device__ __forceinline__ float acc_shaded(float acc, float c, float sh) { // acc += (double)c * sh in double, stored to float
-    return __double2float_rn(__dadd_rn((double)acc, __dmul_rn((double)c, (double)sh)));
+    float out;
+    return cm::acc_shaded_ff(acc, c, sh, out) ? out : acc_shaded_double(acc, c, sh);
 }
 
 __device__ __forceinline__ int gamma_byte(float l, const float* s_gamma) {
@@ -192,10 +204,10 @@ __global__ void __launch_bounds__(kColorThreads) k_colorize(ColorLaunch a) {
     const float* __restrict__ values = a.values;
     const float* __restrict__ aux = a.aux;
     const int ss = a.ss, ws = a.width * ss, hs = a.height * ss;
-    const long long npix = (long long)a.width * a.height;
+    const unsigned npix = (unsigned)a.width * (unsigned)a.height; // (at most 2^31 - 1)
     int fb = 0;
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(p / a.width), j = (int)(p - (long long)i * a.width);
+    for (unsigned p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
+        const int i = (int)(p / (unsigned)a.width), j = (int)(p - (unsigned)i * (unsigned)a.width);
         float lr = 0.0f, lg = 0.0f, lb = 0.0f;
         for (int sa = 0; sa < ss; ++sa)
             for (int sb = 0; sb < ss; ++sb) {
@@ -219,7 +231,7 @@ __global__ void __launch_bounds__(kColorThreads) k_colorize(ColorLaunch a) {
                     lb = cm::add(lb, c.z);
                 } else {
                     const float sh = a.shading == MBX_SHADE_NORMAL_MAP ? normal_shade(__ldg(aux + k), a.lx, a.ly, a.lz)
-                                                                       : relief_shade(values, yy, xx, ws, hs, a.relief, a.lx, a.ly, a.lz);
+                                                                       : relief_shade(a, yy, xx, ws, hs);
                     lr = acc_shaded(lr, c.x, sh);
                     lg = acc_shaded(lg, c.y, sh);
                     lb = acc_shaded(lb, c.z, sh);
@@ -346,6 +358,7 @@ int Colorizer::colorize(const mbx_color_params& p, const float* values, const fl
     a.lx = std::cos(p.light_el) * std::cos(p.light_az);
     a.ly = std::cos(p.light_el) * std::sin(p.light_az);
     a.lz = std::sin(p.light_el);
+    a.relief_ff = cm::ReliefParams{cm::ff_from(a.relief), cm::ff_from(a.lx), cm::ff_from(a.ly), cm::ff_from(a.lz)};
     a.tables = d_tables_;
     a.fallbacks = d_fallbacks_;
     cudaError_t e = cudaMemsetAsync(d_fallbacks_, 0, sizeof(unsigned), st);

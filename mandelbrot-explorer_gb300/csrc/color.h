@@ -35,6 +35,7 @@ struct ColorLaunch {
     int mapping, shading;
     float density;
     double relief, de_k, lx, ly, lz;
+    cm::ReliefParams relief_ff;  // relief, lx, ly, lz as pairs of floats
     const ColorTables* tables;   // device copy
     unsigned* fallbacks;         // device counter of FP64 fallbacks
 };

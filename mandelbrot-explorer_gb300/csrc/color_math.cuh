@@ -190,13 +190,23 @@ CM_HD bool round_checked(ff v, float rel, float& out) {
 constexpr float kLogRel = 0x1p-44f;  // bound used for log_ff (measured below 2^-45)
 constexpr float kExpRel = 0x1p-44f;  // bound used for exp_ff's own rounding
 
+// The FP64 library functions, called: inlined, part of their FP64 work (64 cycles
+// an instruction) was executed for every sample.
+#if defined(__CUDACC__)
+#define CM_CALL __host__ __device__ __noinline__ inline
+#else
+#define CM_CALL inline
+#endif
+CM_CALL float log_fp64(float x) { return (float)::log((double)x); }
+CM_CALL float pow_fp64(float L, float e) { return (float)::pow((double)L, (double)e); }
+
 // RN(log x) for x >= 2^-126; falls back to the FP64 library function
 // (counted in fallbacks) near a rounding midpoint.
 CM_HD float logf_cr(float x, int& fallbacks) {
     float out;
     if (round_checked(log_ff(x), kLogRel, out)) return out;
     ++fallbacks;
-    return (float)::log((double)x);
+    return log_fp64(x);
 }
 
 // RN(L^e) for L > 0, e >= 0 with L^e finite and normal.
@@ -209,7 +219,72 @@ CM_HD float powf_cr(float L, float e, const Exp2Table& tab, int& fallbacks) {
         if (round_checked(exp_ff(y, tab), add(mul(ay, kLogRel), kExpRel), out)) return out;
     }
     ++fallbacks;
-    return (float)::pow((double)L, (double)e);
+    return pow_fp64(L, e);
+}
+
+// ---- shading in pairs of floats ---------------------------------------------
+// The reference shades in double (render.cpp:47-69, 263-292) and stores floats.
+// On GB300 those doubles were the whole cost of a shaded frame: some 58 FP64
+// instructions a sample (conversions included) of 64 cycles a warp, 1.67 ms for
+// a relief frame of 1920x1080 at 3x3 against 0.2 ms of its log and pow. Pairs of
+// floats settle the rounding to float except near its midpoints, where the
+// caller takes the double path. Both functions return false there (and for NaN
+// or anything out of range), else the float the double expression rounds to.
+CM_HD float rsqrt_approx(float x) {
+#if defined(__CUDA_ARCH__)
+    return rsqrtf(x);
+#else
+    return 1.0f / std::sqrt(x);
+#endif
+}
+CM_HD float fabs_(float x) { return from_bits(bits(x) & 0x7fffffffu); }
+// The float nearest to a normalised pair v > 0 whose absolute error is at most err.
+CM_HD bool round_within(ff v, float err, float& out) {
+    const uint32_t u = bits(v.hi);
+    if (!(u - 0x10000000u < 0x60000000u)) return false; // 2^-95 to 2^97, positive
+    const float ulp = from_bits((u & 0x7f800000u) - (23u << 23));
+    const float half = (v.lo < 0.0f && (u & 0x007fffffu) == 0) ? mul(ulp, 0.25f) : mul(ulp, 0.5f);
+    out = v.hi;
+    return add(fabs_(v.lo), err) < half;
+}
+// (float)((double)acc + (double)c * sh), acc, c, sh >= 0: the product is exact in
+// double; its sum with acc rounds to 53 bits first, which can move it by 2^-53.
+CM_HD bool acc_shaded_ff(float acc, float c, float sh, float& out) {
+    const float p = mul(c, sh), e = fma(c, sh, -p); // exact
+    if (e == 0.0f && acc >= 0.0f) { // a product of a float's width: the double sum of two floats rounds to float as the float sum does
+        out = add(acc, p);
+        return true;
+    }
+    const ff s = two_sum(acc, p);                   // exact
+    const ff v = fast_two_sum(s.hi, add(s.lo, e));  // the small parts' sum rounded: 2^-24 of 2^-24
+    return round_within(v, mul(v.hi, 0x1p-46f), out);
+}
+// The relief shade (float)(0.25 + 0.85 max(0, (nx lx + ny ly + lz) / sqrt(nx^2 +
+// ny^2 + 1))) with (nx, ny) = -(sx, sy) strength. Error below 2^-42 absolute for
+// a light vector of length 1: a few roundings of 2^-46, each of a term of the
+// quotient's size.
+struct ReliefParams {
+    ff strength, lx, ly, lz;
+};
+inline ff ff_from(double x) {
+    const float h = (float)x;
+    return {h, (float)(x - (double)h)};
+}
+CM_HD bool relief_ff(float sx, float sy, const ReliefParams& p, float& out) {
+    const ff nx = ff_mul_f(p.strength, -sx), ny = ff_mul_f(p.strength, -sy);
+    if (!(fabs_(nx.hi) < 1e9f && fabs_(ny.hi) < 1e9f)) return false;
+    const ff n2 = ff_add_f(ff_add(ff_mul(nx, nx), ff_mul(ny, ny)), 1.0f);
+    // 1 / sqrt(n2): from the approximation y, r = 1 - n2 y^2, y (1 + r/2 + 3 r^2/8)
+    const float y = rsqrt_approx(n2.hi);
+    const float yy = mul(y, y);
+    const ff r = ff_add_f(ff_mul(ff{-n2.hi, -n2.lo}, ff{yy, fma(y, y, -yy)}), 1.0f);
+    const ff corr = ff_add_f(ff{mul(r.hi, 0.5f), mul(r.lo, 0.5f)}, mul(mul(r.hi, r.hi), 0.375f));
+    const ff inv = ff_add_f(ff_mul_f(corr, y), y);
+    ff d = ff_mul(ff_add(ff_add(ff_mul(nx, p.lx), ff_mul(ny, p.ly)), p.lz), inv);
+    if (d.hi < 0.0f) d = ff{0.0f, 0.0f};
+    // 0.85 = 0x1.b33334p-1 - 0x1.99999ap-26 (to 2^-51)
+    const ff v = ff_add_f(ff_mul(d, ff{0x1.b33334p-1f, -0x1.99999ap-26f}), 0.25f);
+    return round_within(v, 0x1p-42f, out);
 }
 
 } // namespace cm
