@@ -8,6 +8,7 @@
 #include "direct_loop.cuh"
 #include "kernels.h"
 #include "orbit_color.h"
+#include "smooth.cuh"
 
 #include <type_traits>
 
@@ -42,8 +43,20 @@ __device__ __forceinline__ int warp_take(const DeviceFrame& f, int n, int lanes)
     return __shfl_sync(mask, base, 0);
 }
 
-__device__ __forceinline__ double smooth_value(int n, double zrad) {
-    return (double)n - log(log(zrad) / 2 / kLn2) / kLn2;
+__device__ __noinline__ double smooth_value(int n, double zrad) { return (double)n - log(log(zrad) / 2 / kLn2) / kLn2; }
+// (float)smooth_value and the distance as a float: mostly without FP64 (smooth.cuh)
+__device__ __forceinline__ float smooth_float(int n, double zrad) {
+    float v;
+    return smooth_pair(n, zrad, v) ? v : (float)smooth_value(n, zrad);
+}
+__device__ __noinline__ double distance_value(double zrad, double a, double b) { return sqrt(zrad) * log(zrad) / sqrt(a * a + b * b); }
+__device__ __noinline__ float julia_distance(double zrad, double a, double b) {
+    const double denom = sqrt((a * a) + (b * b));
+    return denom > 0.0 ? (float)(sqrt(zrad) * log(zrad) / denom) : 0.0f;
+}
+__device__ __forceinline__ float distance_float(double zrad, double a, double b) {
+    float v;
+    return distance_pair(zrad, a, b, v) ? v : (float)distance_value(zrad, a, b);
 }
 
 // ---------------------------------------------------------------------------
@@ -288,7 +301,7 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
             if (g.ede) {
                 v = (float)(sqrt(zrad) / g.dxf * log(zrad) / sqrt(dr * dr + di * di));
             } else {
-                v = (float)smooth_value(j + 1, zrad);
+                v = smooth_float(j + 1, zrad);
                 if (g.normal) {
                     // normal angle arg(z) - arg(dz/dc) (mp.cpp:2489-2492)
                     if (f.out.normal) f.out.normal[idx] = (float)(atan2(zi, zr) - atan2(di, dr));
@@ -495,10 +508,14 @@ __device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int
 }
 
 struct PixOut {
-    float value;
+    float value; // (interior samples, and the orbit colourings' escapes)
     float nrm;
     int n;
     int state; // 1 escaped, 2 interior, 4 cancelled
+    // at the escape, for the value (fe_escape_value: formed after the loop, by the
+    // warp's samples together)
+    double zrad, zr, zi, jr, ji;
+    FE SJ;
 };
 
 // The plain delta step of pixelRescaled in the fused form, w' = (2 X + s w) w + d,
@@ -714,24 +731,14 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
         if (d_abs_less(g.ESC2, zrad)) { // zrad > ESC2
             o.n = iter;
             o.state = 1;
-            if (g.ede) {
-                double num = sqrt(zrad) * log(zrad);
-                FE Jmag = fe_mul_d(SJ, sqrt(jr * jr + ji * ji));
-                o.value = (float)fe_to_double(fe_div(fe_from(num), fe_mul(p.dxfe, Jmag)));
-                return o;
-            }
-            if (g.normal) {
-                // normal angle arg(z) - arg(J); SJ > 0 (mp.cpp:3512-3515)
-                o.nrm = (float)(atan2(zi, zr) - atan2(ji, jr));
-            } else if (g.deovl) {
-                double num = sqrt(zrad) * log(zrad);
-                FE Jmag = fe_mul_d(SJ, sqrt(jr * jr + ji * ji));
-                o.nrm = (float)fe_to_double(fe_div(fe_from(num), fe_mul(p.dxfe, Jmag)));
-            } else if (OC) { // trap, else stripe average
+            o.zrad = zrad;
+            o.zr = zr;
+            o.zi = zi;
+            o.jr = jr;
+            o.ji = ji;
+            o.SJ = SJ;
+            if (OC && !g.ede && !g.normal && !g.deovl) // trap, else stripe average
                 o.value = oc.escaped((double)iter - log(log(zrad) / 2.0 / kLn2) / kLn2, zrad, g.ER);
-                return o;
-            }
-            o.value = (float)((double)iter - log(log(zrad) / 2.0 / kLn2) / kLn2);
             return o;
         }
         if (detect) {
@@ -895,7 +902,7 @@ __device__ PixOut pixel_fe_nobla(const DeviceFrame& f, const FeParams& p, FE dcr
         if (actual > g.ESC2) {
             o.n = iteration;
             o.state = 1;
-            o.value = (float)((double)iteration - log(log(actual) / 2.0 / kLn2) / kLn2);
+            o.zrad = actual;
             return o;
         }
         if (delta > 1e16 || (delta < 1e-16 && delta > 0.0)) {
@@ -934,6 +941,26 @@ __device__ PixOut pixel_fe_nobla(const DeviceFrame& f, const FeParams& p, FE dcr
     }
 }
 
+// The escaped sample's value, and its normal angle or overlay distance
+// (mp.cpp:3498-3529).
+__device__ __noinline__ float fe_distance(FE dxfe, double zrad, FE SJ, double jr, double ji) {
+    const double num = sqrt(zrad) * log(zrad);
+    const FE Jmag = fe_mul_d(SJ, sqrt(jr * jr + ji * ji));
+    return (float)fe_to_double(fe_div(fe_from(num), fe_mul(dxfe, Jmag)));
+}
+__device__ __forceinline__ void fe_escape_value(const FeParams& p, PixOut& o) {
+    const FrameGeom& g = p.g;
+    if (g.ede) {
+        o.value = fe_distance(p.dxfe, o.zrad, o.SJ, o.jr, o.ji);
+        return;
+    }
+    if (g.normal) // normal angle arg(z) - arg(J); SJ > 0 (mp.cpp:3512-3515)
+        o.nrm = (float)(atan2(o.zi, o.zr) - atan2(o.ji, o.jr));
+    else if (g.deovl)
+        o.nrm = fe_distance(p.dxfe, o.zrad, o.SJ, o.jr, o.ji);
+    o.value = smooth_float(o.n, o.zrad);
+}
+
 template <int OC>
 __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
     if (p.lanes_per_warp && (int)(threadIdx.x & 31u) >= p.lanes_per_warp) return;
@@ -957,6 +984,7 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
         // (the no-BLA lane kernel has no orbit colourings, mp.cpp:2148)
         PixOut o = (OC == 0 && p.no_bla_kernel) ? pixel_fe_nobla(f, p, Dcr, Dci, n_steps) : pixel_fe<OC>(f, p, Dcr, Dci, n_steps, n_bla, n_skip);
         if (o.state == 4) continue; // cancelled
+        if (o.state == 1 && (OC == 0 || g.ede || g.normal || g.deovl)) fe_escape_value(p, o);
         const int idx = sample_index(g, arr);
         // mp.cpp:2173-2183: EMPTY or cutoff-sensitive results go to the
         // arbitrary-precision recompute, flagged here for the host.
@@ -1117,17 +1145,11 @@ __device__ __forceinline__ void direct_write(const DeviceFrame& f, const Shallow
         float v = -2.0f;
         if (!inside) {
             if (g.ede) {
-                const double num = sqrt(d.zrad) * log(d.zrad);
-                if (d.n == 0) {
-                    v = (float)num;
-                } else {
-                    const double denom = sqrt((d.a * d.a) + (d.b * d.b));
-                    v = denom > 0.0 ? (float)(num / denom) : 0.0f;
-                }
+                if (d.n == 0) v = (float)distance_value(d.zrad, 1.0, 0.0);
+                else if (!distance_pair(d.zrad, d.a, d.b, v)) v = julia_distance(d.zrad, d.a, d.b);
                 if (v >= 0.0f) v /= (float)p.dx;
             } else {
-                const double x = log(log(d.zrad) / 2 / kLn2) / kLn2;
-                v = d.n == 0 ? (float)(-x) : (float)((double)d.n - x);
+                v = d.n == 0 ? (float)(-log(log(d.zrad) / 2 / kLn2) / kLn2) : smooth_float(d.n, d.zrad);
             }
         }
         f.out.iter[idx] = v;
@@ -1145,20 +1167,18 @@ __device__ __forceinline__ void direct_write(const DeviceFrame& f, const Shallow
         }
     }
     if (!inside && !((OC & kOcTrap) && !(g.ede || g.normal || g.deovl))) {
-        const bool distance = g.ede || (g.deovl && !g.normal);
-        const double dist = distance ? sqrt(d.zrad) * log(d.zrad) / sqrt(d.a * d.a + d.b * d.b) : 0.0;
         if (g.ede) {
-            val = dist;
+            val = (double)distance_float(d.zrad, d.a, d.b);
         } else {
             if (g.normal) de = atan2(d.zi, d.zr) - atan2(d.b, d.a); // mp.cpp:375-378
-            else if (g.deovl) de = dist;
+            else if (g.deovl) de = distance_value(d.zrad, d.a, d.b);
             if (OC == kOcStripe && !g.normal && !g.deovl) {
                 double cr, ci;
                 direct_c(f, p, arr, cr, ci);
                 const int k = stripe_mark(d.n);
                 val = k > 0 ? shallow_stripe(cr, ci, d.a, d.b, k, d.n, d.zrad, g.ER) : shallow_stripe(cr, ci, cr, ci, 0, d.n, d.zrad, g.ER);
             } else {
-                val = smooth_value(d.n, d.zrad);
+                val = (double)smooth_float(d.n, d.zrad);
             }
         }
     }
