@@ -9,6 +9,8 @@
 #pragma once
 #include <math.h>
 
+#include <cuda_runtime.h>
+
 #include "floatexp.h"
 
 namespace mbx {
@@ -81,6 +83,64 @@ MBX_HD bool operator<=(df32 a, df32 b) { return !(b < a); }
 MBX_HD bool operator>=(df32 a, df32 b) { return !(a < b); }
 MBX_HD bool operator==(df32 a, df32 b) { return a.hi == b.hi && a.lo == b.lo; }
 MBX_HD bool operator!=(df32 a, df32 b) { return !(a == b); }
+
+// Complex double-floats, real and imaginary part side by side: Blackwell's paired
+// FP32 instructions take both parts' operations at once. Each part goes through
+// the operations of operator+ and operator* above in their order (a difference
+// a - b as fma(b, -1, a), one rounding), so the bits are those of the scalar
+// forms; half the instructions matter because the lanes that use them wait for
+// instruction fetch.
+struct cdf {
+    float2 hi, lo;
+};
+MBX_HD cdf cd_make(df32 r, df32 i) { return cdf{make_float2(r.hi, i.hi), make_float2(r.lo, i.lo)}; }
+MBX_HD df32 cd_re(cdf z) { return df32(z.hi.x, z.lo.x); }
+MBX_HD df32 cd_im(cdf z) { return df32(z.hi.y, z.lo.y); }
+MBX_HD float2 f2_add(float2 a, float2 b) {
+#ifdef __CUDA_ARCH__
+    return __fadd2_rn(a, b);
+#else
+    return make_float2(a.x + b.x, a.y + b.y);
+#endif
+}
+MBX_HD float2 f2_mul(float2 a, float2 b) {
+#ifdef __CUDA_ARCH__
+    return __fmul2_rn(a, b);
+#else
+    return make_float2(a.x * b.x, a.y * b.y);
+#endif
+}
+MBX_HD float2 f2_fma(float2 a, float2 b, float2 c) {
+#ifdef __CUDA_ARCH__
+    return __ffma2_rn(a, b, c);
+#else
+    return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
+#endif
+}
+MBX_HD float2 f2_sub(float2 a, float2 b) { return f2_fma(b, make_float2(-1.0f, -1.0f), a); }
+MBX_HD cdf cd_fast_two_sum(float2 a, float2 b) {
+    const float2 s = f2_add(a, b);
+    return cdf{s, f2_sub(b, f2_sub(s, a))};
+}
+MBX_HD cdf operator+(cdf a, cdf b) {
+    const float2 s = f2_add(a.hi, b.hi), t = f2_sub(s, a.hi);
+    const float2 e = f2_add(f2_sub(a.hi, f2_sub(s, t)), f2_sub(b.hi, t));
+    return cd_fast_two_sum(s, f2_add(e, f2_add(a.lo, b.lo)));
+}
+// part by part
+MBX_HD cdf cd_mul(cdf a, cdf b) {
+    const float2 p = f2_mul(a.hi, b.hi);
+    float2 e = f2_fma(a.hi, b.hi, f2_mul(p, make_float2(-1.0f, -1.0f)));
+    e = f2_fma(a.hi, b.lo, f2_fma(a.lo, b.hi, e));
+    return cd_fast_two_sum(p, e);
+}
+MBX_HD cdf cd_scale(df32 a, cdf b) { return cd_mul(cd_make(a, a), b); }
+// (ar br - ai bi, ar bi + ai br)
+MBX_HD cdf cd_cmul(df32 ar, df32 ai, cdf b) {
+    const cdf i{make_float2(-b.hi.y, b.hi.x), make_float2(-b.lo.y, b.lo.x)};
+    return cd_scale(ar, b) + cd_scale(ai, i);
+}
+MBX_HD cdf cd_twice(cdf a) { return cdf{f2_add(a.hi, a.hi), f2_add(a.lo, a.lo)}; }
 
 MBX_DF_CALL df32 tsqrt(df32 a) {
     if (!(a.hi > 0.0f)) return df32(0.0f);

@@ -624,8 +624,8 @@ cudaError_t Engine::run_df_pass(const DeviceFrame& f) {
     // the queue length is known only on the device: both widths are launched
     // and the one it selects runs
     p.wide_from = kWideLanesPerSm * (unsigned)nsm_;
-    auto narrow = p.g.deriv ? k_lane_pass<df32, 128, 2, 8, true, false, true> : k_lane_pass<df32, 128, 2, 8>;
-    auto wide = p.g.deriv ? k_lane_pass<df32, 128, 2, 32, true, false, true> : k_lane_pass<df32, 128, 2, 32>;
+    auto narrow = p.g.deriv ? k_lane_pass<df32, 128, 3, 8, true, false, true> : k_lane_pass<df32, 128, 3, 8>;
+    auto wide = p.g.deriv ? k_lane_pass<df32, 128, 3, 32, true, false, true> : k_lane_pass<df32, 128, 3, 32>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -646,8 +646,8 @@ cudaError_t launch_batch_pass(int tier, const BatchArgs& a, int nsm, cudaStream_
         BatchArgs b = a;
         b.wide_from = kWideLanesPerSm * (unsigned)nsm;
         if (a.deriv) {
-            k_batch_pass<df32, 128, 2, 8, true><<<nsm * 4, 128, 0, st>>>(b);
-            k_batch_pass<df32, 128, 2, 32, true><<<nsm * 4, 128, 0, st>>>(b);
+            k_batch_pass<df32, 128, 3, 8, true><<<nsm * 4, 128, 0, st>>>(b);
+            k_batch_pass<df32, 128, 3, 32, true><<<nsm * 4, 128, 0, st>>>(b);
         } else {
             // 128 registers without spills: four blocks of 128 per SM (a
             // batch's queue holds many waves of samples; measured on 24

@@ -437,17 +437,29 @@ MBX_HDF int lane_bla(const BlaView& b, const BlaEntry<T>* t, const typename Lane
         const int land = s + l;
         if (land >= mx_ref_it - 1) continue;
         // A dz + B dc = A (S.m w) 2^(ea + S.e) + B dcm 2^(eb + dce)
-        const T swr = S.m * wr, swi = S.m * wi;
-        T t1r = e.ar * swr - e.ai * swi, t1i = e.ar * swi + e.ai * swr;
-        T t2r = e.br * dcm.x - e.bi * dcm.y, t2i = e.br * dcm.y + e.bi * dcm.x;
         const int E1 = e.ea + S.e, E2 = e.eb + dce;
         const int E = imax(E1, E2);
-        const T vr = ldexp_ftz(t1r, E1 - E) + ldexp_ftz(t2r, E2 - E);
-        const T vi = ldexp_ftz(t1i, E1 - E) + ldexp_ftz(t2i, E2 - E);
+        const typename LaneReal<T>::V2 zl = orb[land];
+        T vr, vi, zr, zi;
+        if constexpr (std::is_same<T, df32>::value) {
+            const cdf t1 = cd_cmul(e.ar, e.ai, cd_scale(S.m, cd_make(wr, wi))), t2 = cd_cmul(e.br, e.bi, cd_make(dcm.x, dcm.y));
+            const cdf v = cd_make(ldexp_ftz(cd_re(t1), E1 - E), ldexp_ftz(cd_im(t1), E1 - E)) + cd_make(ldexp_ftz(cd_re(t2), E2 - E), ldexp_ftz(cd_im(t2), E2 - E));
+            vr = cd_re(v);
+            vi = cd_im(v);
+            const cdf z = cd_make(zl.x, zl.y) + cd_make(ldexp_ftz(vr, E), ldexp_ftz(vi, E));
+            zr = cd_re(z);
+            zi = cd_im(z);
+        } else {
+            const T swr = S.m * wr, swi = S.m * wi;
+            T t1r = e.ar * swr - e.ai * swi, t1i = e.ar * swi + e.ai * swr;
+            T t2r = e.br * dcm.x - e.bi * dcm.y, t2i = e.br * dcm.y + e.bi * dcm.x;
+            vr = ldexp_ftz(t1r, E1 - E) + ldexp_ftz(t2r, E2 - E);
+            vi = ldexp_ftz(t1i, E1 - E) + ldexp_ftz(t2i, E2 - E);
+            zr = zl.x + ldexp_ftz(vr, E);
+            zi = zl.y + ldexp_ftz(vi, E);
+        }
         const T v2 = vr * vr + vi * vi;
         // Never skip past an escape: z = X_land + dz' (conservative test).
-        const typename LaneReal<T>::V2 zl = orb[land];
-        const T zr = zl.x + ldexp_ftz(vr, E), zi = zl.y + ldexp_ftz(vi, E);
         if (R::zabs2(zr, zi) > ESC2lo) return 0;
         if (v2 == T(0)) {
             if (!periodic) return 0;
@@ -544,7 +556,10 @@ MBX_HD typename LaneReal<T>::V2 lane_d(T Sm, int k, typename LaneReal<T>::V2 dcm
     const T inv = fdiv_approx(T(1), Sm);
     return LaneReal<T>::make2(ldexp_ftz(dcm.x * inv, k), ldexp_ftz(dcm.y * inv, k));
 }
-MBX_RARE df2 lane_d_df(df32 Sm, int k, df2 dcm) { return lane_d<df32>(Sm, k, dcm); }
+MBX_RARE df2 lane_d_df(df32 Sm, int k, df2 dcm) {
+    const cdf d = cd_scale(df32(1.0f) / Sm, cd_make(dcm.x, dcm.y));
+    return df2{ldexp_ftz(cd_re(d), k), ldexp_ftz(cd_im(d), k)};
+}
 template <class T>
 MBX_HD void lane_refresh(Lane<T>& L) {
     L.s = te_to_real(L.S);
@@ -630,10 +645,16 @@ MBX_HD void lane_j_window(Lane<T>& L) {
 // J' = 2 z J + 1 with z at unit scale in the lane type.
 template <class T>
 MBX_HD void lane_j_step(Lane<T>& L, T zr, T zi) {
-    const T a = lane_twice(zr * L.jr - zi * L.ji) + L.invSJ;
-    const T b = lane_twice(zr * L.ji + zi * L.jr);
-    L.jr = a;
-    L.ji = b;
+    if constexpr (std::is_same<T, df32>::value) {
+        const cdf j = cd_twice(cd_cmul(zr, zi, cd_make(L.jr, L.ji)));
+        L.jr = cd_re(j) + L.invSJ;
+        L.ji = cd_im(j);
+    } else {
+        const T a = lane_twice(zr * L.jr - zi * L.ji) + L.invSJ;
+        const T b = lane_twice(zr * L.ji + zi * L.jr);
+        L.jr = a;
+        L.ji = b;
+    }
     lane_j_window(L);
 }
 // The FP32 lane's form, from 2 z = 2 X + 2 s w as the common-step loop forms it.
@@ -854,6 +875,16 @@ MBX_HD void lane_step<float>(float2 X, float s, float wr, float wi, float dr, fl
     nwi = fmaf(f.x, wi, fmaf(f.y, wr, di));
     const float wm2 = fmaf(nwr, nwr, nwi * nwi);
     nerr2 = fmaf(err2, g2, LaneReal<float>::kEps2 * wm2);
+}
+
+// The double-float step in paired operations (the generic form's, part by part).
+template <>
+MBX_HD void lane_step<df32>(df2 X, df32 s, df32 wr, df32 wi, df32 dr, df32 di, float err2, float g2, df32& nwr, df32& nwi, float& nerr2) {
+    const cdf w = cd_make(wr, wi), f = cd_twice(cd_make(X.x, X.y)) + cd_scale(s, w);
+    const cdf n = cd_cmul(cd_re(f), cd_im(f), w) + cd_make(dr, di);
+    nwr = cd_re(n);
+    nwi = cd_im(n);
+    nerr2 = err2 * g2 + LaneReal<df32>::kEps2 * (nwr.hi * nwr.hi + nwi.hi * nwi.hi);
 }
 
 // z = X + s w (per component); as one FMA in the FP32 lane.
@@ -1304,12 +1335,10 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                 // the double-float lane carries s w: z = X + s w now and
                 // f = 2 X + s w of the next step take the same product, and J's
                 // pre-step z is the z of the step before
-                T tr = T(0), ti = T(0), zpr = T(0), zpi = T(0);
-                if constexpr (!std::is_same<T, float>::value) {
-                    tr = L.s * L.wr;
-                    ti = L.s * L.wi;
-                    zpr = L.Xc.x + tr;
-                    zpi = L.Xc.y + ti;
+                cdf t{}, zp{};
+                if constexpr (std::is_same<T, df32>::value) {
+                    t = cd_scale(L.s, cd_make(L.wr, L.wi));
+                    zp = cd_make(L.Xc.x, L.Xc.y) + t;
                 }
                 for (;;) {
                     if (m >= mlim) break;
@@ -1335,21 +1364,23 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                     const typename R::V2 X = orb[nrm];
                     T nwr, nwi;
                     E nerr2;
-                    T zr, zi, ntr, nti;
+                    T zr, zi;
+                    cdf nt{}, z{};
                     if constexpr (std::is_same<T, float>::value) {
                         lane_step<T>(L.Xc, L.s, L.wr, L.wi, L.dr, L.di, L.err2, L.g2, nwr, nwi, nerr2);
                         zr = lane_zc<T>(X.x, L.s, nwr);
                         zi = lane_zc<T>(X.y, L.s, nwi);
                     } else { // lane_step and lane_zc
-                        const T fR = lane_twice(L.Xc.x) + tr, fI = lane_twice(L.Xc.y) + ti;
-                        nwr = fR * L.wr - fI * L.wi + L.dr;
-                        nwi = fR * L.wi + fI * L.wr + L.di;
+                        const cdf f = cd_twice(cd_make(L.Xc.x, L.Xc.y)) + t;
+                        const cdf n = cd_cmul(cd_re(f), cd_im(f), cd_make(L.wr, L.wi)) + cd_make(L.dr, L.di);
+                        nwr = cd_re(n);
+                        nwi = cd_im(n);
                         const E a = R::toe(nwr), c = R::toe(nwi);
                         nerr2 = L.err2 * L.g2 + R::kEps2 * (a * a + c * c);
-                        ntr = L.s * nwr;
-                        nti = L.s * nwi;
-                        zr = X.x + ntr;
-                        zi = X.y + nti;
+                        nt = cd_scale(L.s, n);
+                        z = cd_make(X.x, X.y) + nt;
+                        zr = cd_re(z);
+                        zi = cd_im(z);
                     }
                     const Z zrad = R::zabs2(zr, zi);
                     const Z wm2 = R::zabs2(nwr, nwi);
@@ -1363,12 +1394,10 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                         if (deriv) lane_j_advance(L); // (from the pre-step state)
                     } else {
                         if (deriv) {
-                            lane_j_step(L, zpr, zpi);
-                            zpr = zr;
-                            zpi = zi;
+                            lane_j_step(L, cd_re(zp), cd_im(zp));
+                            zp = z;
                         }
-                        tr = ntr;
-                        ti = nti;
+                        t = nt;
                     }
                     L.wr = nwr;
                     L.wi = nwi;
@@ -1529,7 +1558,15 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
             wrapped = sync;
         }
         L.Xc = orb[L.rm];
-        const T zr = lane_zc<T>(L.Xc.x, L.s, L.wr), zi = lane_zc<T>(L.Xc.y, L.s, L.wi);
+        T zr, zi;
+        if constexpr (std::is_same<T, df32>::value) {
+            const cdf z = cd_make(L.Xc.x, L.Xc.y) + cd_scale(L.s, cd_make(L.wr, L.wi));
+            zr = cd_re(z);
+            zi = cd_im(z);
+        } else {
+            zr = lane_zc<T>(L.Xc.x, L.s, L.wr);
+            zi = lane_zc<T>(L.Xc.y, L.s, L.wi);
+        }
         const Z zrad = R::zabs2(zr, zi);
         if (zrad > ESC2lo) {
             Z zesc = zrad;
