@@ -1784,6 +1784,11 @@ int Engine::run_pass(std::vector<uint64_t>* keys, const PixelSet& grid, int mx_r
     stats_.effective_iterations += (long long)hctr_->effective_iters;
     stats_.interior += (int)hctr_->interior;
     stats_.samples += n;
+    if (hctr_->finished == (unsigned)n && hctr_->gmp_flags == 0) { // every entry has its value: no flags to read
+        if (have_new_ref) *have_new_ref = false;
+        if (keys) keys->clear();
+        return MBX_OK;
+    }
     // Pending entries, arbitrary-precision recomputes and the next reference.
     hdone_.resize(n);
     hgmp_.resize(n);

@@ -276,4 +276,65 @@ MBX_HD C2 c_div(C2 num, C2 den) {
     return c2(x, y);
 }
 
+// c_div by one denominator many times (the series-approximation seeds: up to 30
+// divisions a sample). The ratio and the scaled denominator of Smith's algorithm
+// are formed once, and each quotient by the denominator comes from its correctly
+// rounded reciprocal y: q = a y, then twice q += (a - q denom) y with fused
+// operations; after the first q is faithful, and then the second rounds
+// correctly (Markstein's theorem, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", 1990): the bits of c_div's division in 5 FP64
+// instructions for about 9. Numerators or quotients near the ends of the range,
+// or a denominator whose mantissa is all ones, take c_div.
+struct CDivBy {
+    C2 den;
+    double ratio, denom, y;
+    bool swap, scale, ok;
+};
+MBX_HD double d_fma(double a, double b, double c) {
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, b, c);
+#else
+    return __builtin_fma(a, b, c);
+#endif
+}
+// the exponent within [2^-400, 2^400]: no quotient or residual of two leaves the range
+MBX_HD bool d_mid(double x) { return (unsigned)((dbits(x) >> 52) & 0x7ff) - 623u <= 800u; }
+MBX_HD CDivBy c_div_by(C2 den) {
+    CDivBy q;
+    q.den = den;
+    q.swap = d_abs_less(den.re, den.im);
+    double c = den.re, d = den.im;
+    const double big = q.swap ? d : c;
+    q.scale = d_abs_less(big, 2.2204460492503130808e-16);
+    if (q.scale) {
+        c = c * 4503599627370496.0;
+        d = d * 4503599627370496.0;
+    }
+    q.ratio = q.swap ? c / d : d / c;
+    q.denom = q.swap ? (c * q.ratio) + d : (d * q.ratio) + c;
+    q.y = 1.0 / q.denom;
+    q.ok = d_mid(big) && d_mid(q.denom) && d_abs_less(2.2250738585072013831e-308, q.ratio) && (dbits(q.denom) & 0xfffffffffffffull) != 0xfffffffffffffull;
+    return q;
+}
+MBX_HD double d_quotient(double a, double b, double y) {
+    double q = a * y;
+    q = d_fma(d_fma(-q, b, a), y, q);
+    return d_fma(d_fma(-q, b, a), y, q);
+}
+MBX_COLD C2 c_div_rare(C2 num, C2 den) { return c_div(num, den); }
+MBX_HD C2 c_div(C2 num, const CDivBy& by) {
+    double a = num.re, b = num.im;
+    if (by.ok && d_mid(a) && d_mid(b)) {
+        if (by.scale) {
+            a = a * 4503599627370496.0;
+            b = b * 4503599627370496.0;
+        }
+        // the numerators of c_div's two quotients
+        const double xn = by.swap ? (a * by.ratio) + b : (b * by.ratio) + a;
+        const double yn = by.swap ? (b * by.ratio) - a : b - (a * by.ratio);
+        if (d_mid(xn) && d_mid(yn)) return c2(d_quotient(xn, by.denom, by.y), d_quotient(yn, by.denom, by.y));
+    }
+    return c_div_rare(num, by.den);
+}
+
 } // namespace mbx

@@ -123,7 +123,7 @@ struct Counters {
     unsigned long long glitch_min_bits;  // min glitch score (as non-negative double bits)
     unsigned long long effective_iters;  // sum of N (maxiter for interior)
     unsigned int rerun_n;                // mixed pass: entries queued for the FP64 floatexp pass
-    unsigned int finished;               // mixed pass: entries finished or queued
+    unsigned int finished;               // entries finished (mixed pass: or queued)
     unsigned int gmp_flags;              // floatexp pass: entries flagged for the arbitrary-precision recompute
     unsigned int interior_flagged;       // lane passes: interior decisions queued for the next tier
     unsigned int escape_flagged;         // lane passes: escapes queued for the next tier (|z|^2 too near the bailout for the estimate)
@@ -161,6 +161,7 @@ struct Fp64Params {
     int mx_ref_it;
     int use_interior, int_rep, interior_confirm;
     double interior_eps2;
+    unsigned esc_word = 0;   // direct_escape_word(g.ESC2), set by launch_fp64_pass
 };
 
 // Floatexp rescaled loop parameters (mp.cpp:3287-3618, 3620-3816).

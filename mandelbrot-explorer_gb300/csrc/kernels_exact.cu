@@ -59,11 +59,16 @@ __device__ __forceinline__ float distance_float(double zrad, double a, double b)
     return distance_pair(zrad, a, b, v) ? v : (float)distance_value(zrad, a, b);
 }
 
+// High words of a part's magnitude that settle a step's tests without FP64:
+// from kFeNearWord (just above 1e-4) on, |z|^2 >= 1e-8; in [kFeWLo, kFeWHi)
+// (just above 1e-8, 7e7) the larger part of w keeps |w|^2 within [1e-16, 1e16].
+constexpr unsigned kFeNearWord = 0x3f1a36e3u, kFeWLo = 0x3e45798fu, kFeWHi = 0x4190b076u;
+
 // ---------------------------------------------------------------------------
 // Double path (mp.cpp:2290-2585, tryBLA mp.cpp:2714-2755).
-__device__ __forceinline__ int bla_try_fp64(const BlaView& b, const double2* Z, int s, double& dzr, double& dzi, double& ddr, double& ddi, double dcr, double dci, bool ede, double ESC2, int mx_ref_it) {
-    if (s < 1 || b.nlev == 0) return 0;
-    double zmag2 = dzr * dzr + dzi * dzi;
+// zmag2: |dz|^2
+__device__ __forceinline__ int bla_try_fp64(const BlaView& b, const double2* Z, int s, double zmag2, double& dzr, double& dzi, double& ddr, double& ddi, double dcr, double dci, bool ede, double ESC2,
+                                            int mx_ref_it) {
     int maxp = b.nlev - 1;
     int startp = (s == 1) ? maxp : __ffs(s - 1) - 1;
     if (startp > maxp) startp = maxp;
@@ -71,8 +76,8 @@ __device__ __forceinline__ int bla_try_fp64(const BlaView& b, const double2* Z, 
     for (int p = startp; p >= b.minlevel; --p) {
         int i = (s - 1) >> p;
         if (i >= b.size[p]) continue;
-        double r2 = b.r2[b.off[p] + i];
-        if (r2 <= 0 || zmag2 >= r2) continue;
+        const double r2 = b.r2[b.off[p] + i];
+        if (!d_abs_less(zmag2, r2)) continue; // (r2 >= +0)
         int l = 1 << p;
         int land = s + l;
         if (land >= mx_ref_it - 1) continue;
@@ -81,7 +86,7 @@ __device__ __forceinline__ int bla_try_fp64(const BlaView& b, const double2* Z, 
         double nzi = bc.x * dzi + bc.y * dzr + bc.z * dci + bc.w * dcr;
         double2 zl = Z[land];
         double fr = zl.x + nzr, fi = zl.y + nzi;
-        if (fr * fr + fi * fi > ESC2) return 0;
+        if (d_abs_less(ESC2, fr * fr + fi * fi)) return 0; // > ESC2
         if (ede) {
             double4 bd = b.ce[b.off[p] + i];
             double nddr = (bd.x * dzr - bd.y * dzi) + (bc.x * ddr - bc.y * ddi) + (bd.z * dcr - bd.w * dci);
@@ -104,8 +109,10 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
     const FrameGeom& g = p.g;
     const double2* Z = f.orbit.Z;
     const double2* D = f.orbit.D;
+    const CDivBy by_delta = c_div_by(p.sa_delta);
+    const int bla_mask = (1 << f.bla.minlevel) - 1;
     unsigned long long n_steps = 0, n_bla = 0, n_skip = 0, n_eff = 0;
-    unsigned int n_int = 0;
+    unsigned int n_int = 0, n_fin = 0;
     for (;;) {
         const int first = warp_take(f, f.px.n, 32);
         if (first < 0) break;
@@ -123,18 +130,19 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
         for (int x = p.sa_order; x >= 0; --x) {
             dz = c_add(dz, p.A[x]);
             dz = c_mul(dz, dc);
-            dz = c_div(dz, p.sa_delta);
+            dz = c_div(dz, by_delta);
         }
         if (g.deriv) {
             for (int x = p.sa_order; x >= 0; --x) {
                 dd = c_add(dd, p.B[x]);
                 dd = c_mul(dd, dc);
-                dd = c_div(dd, p.sa_delta);
+                dd = c_div(dd, by_delta);
             }
         }
         int j = p.sa_it + 1;
         double dzr = dz.re, dzi = dz.im, dcr = dc.re, dci = dc.im, ddr = dd.re, ddi = dd.im;
-        double tmp, zr = 0, zi = 0, dr = 0, di = 0, zrad = 0;
+        double tmp, zr = 0, zi = 0, zrad = 0;
+        double q_r = dzr * dzr, q_i = dzi * dzi; // dz's squares, kept with it
         int k = j;
         const int per = p.per;
         int rk = k, rkm1 = k - 1;
@@ -149,6 +157,7 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
         double sdzr = 1e300, sdzi = 1e300;
         int sk = -1, save_j2 = j, twin2 = 1;
         int outcome = 0; // 0 running, 1 escaped, 2 interior, 3 glitch
+        double edr = 0, edi = 0; // dz/dc at the escape
         double gscore = -1.0;
         int tick = 0;
         while (j < g.mxit) {
@@ -157,7 +166,7 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
                 break;
             }
             if (int_rep) {
-                if (k == sk && dzr == sdzr && dzi == sdzi) {
+                if (k == sk && d_eq(dzr, sdzr) && d_eq(dzi, sdzi)) {
                     outcome = 2;
                     break;
                 }
@@ -169,8 +178,10 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
                     twin2 += twin2;
                 }
             }
-            if (f.bla.use && !(OC & kOcTrap) && dzr * dzr + dzi * dzi < f.bla.rmax2) {
-                int skip = bla_try_fp64(f.bla, Z, rkm1, dzr, dzi, ddr, ddi, dcr, dci, g.deriv, g.ESC2, p.mx_ref_it);
+            // (a BLA position: the orbit index less one a multiple of the least skip)
+            const double q = rkm1 >= 1 && ((rkm1 - 1) & bla_mask) == 0 && f.bla.use && !(OC & kOcTrap) ? q_r + q_i : 1e300;
+            if (d_abs_less(q, f.bla.rmax2)) {
+                int skip = bla_try_fp64(f.bla, Z, rkm1, q, dzr, dzi, ddr, ddi, dcr, dci, g.deriv, g.ESC2, p.mx_ref_it);
                 if (skip > 0) {
                     ++n_bla;
                     n_skip += skip;
@@ -179,6 +190,8 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
                     rk += skip;
                     if (per && rk >= per) rk -= per;
                     rkm1 = (per && rk == 0) ? per - 1 : rk - 1;
+                    q_r = dzr * dzr;
+                    q_i = dzi * dzi;
                     oc.skipped();
                     zsr = 1e30;
                     zsi = 1e30;
@@ -192,33 +205,31 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
             ++n_steps;
             if (g.deriv) {
                 if (k == 0) {
-                    tmp = (dzr * (1 + ddr) - dzi * (1 + ddi)) * 2;
-                    ddi = (dzr * (1 + ddi) + dzi * (1 + ddr)) * 2;
+                    tmp = d_twice(dzr * (1 + ddr) - dzi * (1 + ddi));
+                    ddi = d_twice(dzr * (1 + ddi) + dzi * (1 + ddr));
                 } else {
                     double2 zk = Z[k - 1], dk = D[k - 1];
-                    tmp = (ddr * zk.x - ddi * zk.y + dzr * (dk.x + ddr) - dzi * (dk.y + ddi)) * 2;
-                    ddi = (ddr * zk.y + ddi * zk.x + dzr * (dk.y + ddi) + dzi * (dk.x + ddr)) * 2;
+                    tmp = d_twice(ddr * zk.x - ddi * zk.y + dzr * (dk.x + ddr) - dzi * (dk.y + ddi));
+                    ddi = d_twice(ddr * zk.y + ddi * zk.x + dzr * (dk.y + ddi) + dzi * (dk.x + ddr));
                 }
                 ddr = tmp;
-                double2 dk1 = D[k];
-                dr = ddr + dk1.x;
-                di = ddi + dk1.y;
             }
-            double dzr2 = dzr * dzr;
-            double dzi2 = dzi * dzi;
+            const double m = d_twice(dzr * dzi);
             if (k == 0) {
-                tmp = dzr2 - dzi2 + dcr;
-                dzi = dzr * dzi * 2 + dci;
+                tmp = q_r - q_i + dcr;
+                dzi = m + dci;
             } else {
                 double2 zp = Z[rkm1];
-                tmp = (dzr * zp.x - dzi * zp.y) * 2 + dzr2 - dzi2 + dcr;
-                dzi = (dzr * zp.y + dzi * zp.x) * 2 + dzr * dzi * 2 + dci;
+                tmp = d_twice(dzr * zp.x - dzi * zp.y) + q_r - q_i + dcr;
+                dzi = d_twice(dzr * zp.y + dzi * zp.x) + m + dci;
             }
             dzr = tmp;
+            q_r = dzr * dzr;
+            q_i = dzi * dzi;
             double2 zc = Z[rk];
             zr = dzr + zc.x;
             zi = dzi + zc.y;
-            zrad = zr * zr + zi * zi;
+            const int kd = k; // the derivative shadow's entry of this z
             oc.push(zr, zi);
             ++k;
             rkm1 = rk;
@@ -226,7 +237,28 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
                 if (++rk == per) rk = 0;
             } else
                 rk = k;
-            if (zrad > g.ESC2) {
+            // A common iteration, settled on high words: |z| below the bailout and
+            // at least twice |dz|'s larger part (so |z|^2 is not below |dz|^2: no
+            // rebase), the reference not at its end, no interior test due (as in
+            // pixel_fe). 16 FP64 instructions; the tests below formed some 30.
+            const unsigned hz = umax_(hi_abs(zr), hi_abs(zi));
+            if (hz < p.esc_word && hz >= umax_(hi_abs(dzr), hi_abs(dzi)) + 0x00100000u && (per || k != p.mx_ref_it) &&
+                (!detect || (conf_P <= 0 && ((j & 15) != 0 || conf_giveup >= 3 ||
+                                             (hz >= kFeNearWord && j - save_j < period_win && umax_(hi_abs(zr - zsr), hi_abs(zi - zsi)) + 0x01b00000u >= hz &&
+                                              d_abs_less(p.interior_eps2, 1e-17)))))) {
+                ++j;
+                continue;
+            }
+            zrad = zr * zr + zi * zi;
+            double dr = 0, di = 0;
+            if (g.deriv) {
+                const double2 dk1 = D[kd];
+                dr = ddr + dk1.x;
+                di = ddi + dk1.y;
+            }
+            if (d_abs_less(g.ESC2, zrad)) { // zrad > ESC2
+                edr = dr;
+                edi = di;
                 outcome = 1;
                 break;
             }
@@ -270,14 +302,16 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
                     }
                 }
             }
-            if (zrad < dzr * dzr + dzi * dzi || (!per && k == p.mx_ref_it)) {
-                if ((dzr * dzr + dzi * dzi) / zrad > 10000000) {
+            if (d_abs_less(zrad, q_r + q_i) || (!per && k == p.mx_ref_it)) {
+                if ((q_r + q_i) / zrad > 10000000) {
                     gscore = zrad / f.orbit.zm3[per ? j % per : j];
                     outcome = 3;
                     break;
                 }
                 dzr = zr;
                 dzi = zi;
+                q_r = dzr * dzr;
+                q_i = dzi * dzi;
                 if (g.deriv) {
                     ddr = dr - 1;
                     ddi = di;
@@ -299,14 +333,14 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
         if (outcome == 1) {
             float v;
             if (g.ede) {
-                v = (float)(sqrt(zrad) / g.dxf * log(zrad) / sqrt(dr * dr + di * di));
+                v = (float)(sqrt(zrad) / g.dxf * log(zrad) / sqrt(edr * edr + edi * edi));
             } else {
                 v = smooth_float(j + 1, zrad);
                 if (g.normal) {
                     // normal angle arg(z) - arg(dz/dc) (mp.cpp:2489-2492)
-                    if (f.out.normal) f.out.normal[idx] = (float)(atan2(zi, zr) - atan2(di, dr));
+                    if (f.out.normal) f.out.normal[idx] = (float)(atan2(zi, zr) - atan2(edi, edr));
                 } else if (g.deovl) {
-                    if (f.out.normal) f.out.normal[idx] = (float)(sqrt(zrad) / g.dxf * log(zrad) / sqrt(dr * dr + di * di));
+                    if (f.out.normal) f.out.normal[idx] = (float)(sqrt(zrad) / g.dxf * log(zrad) / sqrt(edr * edr + edi * edi));
                 } else if (OC) { // trap, else stripe average (mp.cpp:2497-2500)
                     v = oc.escaped(smooth_value(j + 1, zrad), zrad, g.ER);
                 }
@@ -314,11 +348,13 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
             f.out.iter[idx] = v;
             if (f.out.escN) f.out.escN[idx] = j + 1;
             f.out.done[i] = 1;
+            ++n_fin;
             n_eff += (unsigned long long)(j + 1);
         } else if (outcome == 2) {
             f.out.iter[idx] = oc.interior();
             if (f.out.escN) f.out.escN[idx] = -1;
             f.out.done[i] = 1;
+            ++n_fin;
             n_eff += (unsigned long long)g.mxit;
             ++n_int;
         } else {
@@ -331,6 +367,7 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
     atomicAdd(&f.ctr->bla_skipped, n_skip);
     atomicAdd(&f.ctr->effective_iters, n_eff);
     atomicAdd(&f.ctr->interior, n_int);
+    atomicAdd(&f.ctr->finished, n_fin);
 }
 
 // ---------------------------------------------------------------------------
@@ -534,10 +571,6 @@ __device__ __forceinline__ void fe_plain_step(double Xr, double Xi, double swr, 
     nwr = fR * wr - fI * wi + dr;
     nwi = fR * wi + fI * wr + di;
 }
-// High words of a part's magnitude that settle a step's tests without FP64:
-// from kFeNearWord (just above 1e-4) on, |z|^2 >= 1e-8; in [kFeWLo, kFeWHi)
-// (just above 1e-8, 7e7) the larger part of w keeps |w|^2 within [1e-16, 1e16].
-constexpr unsigned kFeNearWord = 0x3f1a36e3u, kFeWLo = 0x3e45798fu, kFeWHi = 0x4190b076u;
 // |x| < 2^-1056 (the subnormal 2^18 * 2^-1074): the step's underflow test, on
 // the bit pattern
 __device__ __forceinline__ bool below_step_floor(double x) { return (dbits(x) & 0x7fffffffffffffffull) < 0x40000ull; }
@@ -966,7 +999,7 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
     if (p.lanes_per_warp && (int)(threadIdx.x & 31u) >= p.lanes_per_warp) return;
     const FrameGeom& g = p.g;
     unsigned long long n_steps = 0, n_bla = 0, n_skip = 0, n_eff = 0;
-    unsigned int n_int = 0;
+    unsigned int n_int = 0, n_fin = 0;
     const int n = f.px.n_dev ? min((int)*f.px.n_dev, f.px.n) : f.px.n;
     const int lanes = p.lanes_per_warp ? p.lanes_per_warp : 32;
     for (;;) {
@@ -997,6 +1030,7 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
         if ((g.deovl || g.normal) && f.out.normal) f.out.normal[idx] = o.nrm;
         if (f.out.escN) f.out.escN[idx] = o.state == 1 ? o.n : -1;
         f.out.done[i] = 1;
+        ++n_fin;
         if (o.state == 1) {
             n_eff += (unsigned long long)o.n;
         } else {
@@ -1009,6 +1043,7 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
     atomicAdd(&f.ctr->bla_skipped, n_skip);
     atomicAdd(&f.ctr->effective_iters, n_eff);
     atomicAdd(&f.ctr->interior, n_int);
+    atomicAdd(&f.ctr->finished, n_fin);
 }
 
 // ---------------------------------------------------------------------------
@@ -1533,7 +1568,9 @@ cudaError_t launch_fill(float* iter, float* normal, int32_t* escN, size_t n, cud
     k_fill<<<blocks, 256, 0, st>>>(iter, normal, escN, n);
     return cudaGetLastError();
 }
-cudaError_t launch_fp64_pass(const DeviceFrame& f, const Fp64Params& p, int blocks, int threads, cudaStream_t st) {
+cudaError_t launch_fp64_pass(const DeviceFrame& f, const Fp64Params& fp, int blocks, int threads, cudaStream_t st) {
+    Fp64Params p = fp;
+    p.esc_word = direct_escape_word(p.g.ESC2);
     switch (p.g.oc) {
     case 0: k_fp64_pass<0><<<blocks, threads, 0, st>>>(f, p); break;
     case kOcStripe: k_fp64_pass<kOcStripe><<<blocks, threads, 0, st>>>(f, p); break;
