@@ -5,6 +5,7 @@
 //
 // Reference: cbotx/Mandelbrot-Explorer src/engine/mandel_perturbation.cpp
 // ("mp.cpp"); the per-pixel semantics are those of its scalar loops.
+#include "counts.cuh"
 #include "direct_loop.cuh"
 #include "kernels.h"
 #include "orbit_color.h"
@@ -104,8 +105,29 @@ __device__ __forceinline__ int bla_try_fp64(const BlaView& b, const double2* Z, 
 // OC: the orbit colourings (orbit_color.h): their accumulators take every
 // iteration's z; a trap turns BLA and the state-repetition detector off
 // (mp.cpp:2121, 2388), a BLA skip restarts the stripe window (:2422-2427).
+__device__ __forceinline__ void exact_counts(Counters* c, BlockCounts& s, unsigned long long n_steps, unsigned long long n_bla, unsigned long long n_skip, unsigned long long n_eff, unsigned n_int,
+                                             unsigned n_fin, int lanes) {
+    block_count(s, 0, n_steps, lanes);
+    block_count(s, 1, n_bla, lanes);
+    block_count(s, 2, n_skip, lanes);
+    block_count(s, 3, n_eff, lanes);
+    block_count(s, 4, n_int, lanes);
+    block_count(s, 5, n_fin, lanes);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        counts_flush(&c->steps, s.v[0]);
+        counts_flush(&c->bla_applies, s.v[1]);
+        counts_flush(&c->bla_skipped, s.v[2]);
+        counts_flush(&c->effective_iters, s.v[3]);
+        counts_flush(&c->interior, s.v[4]);
+        counts_flush(&c->finished, s.v[5]);
+    }
+}
+
 template <int OC>
 __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) {
+    __shared__ BlockCounts s_counts;
+    block_counts_init(s_counts);
     const FrameGeom& g = p.g;
     const double2* Z = f.orbit.Z;
     const double2* D = f.orbit.D;
@@ -362,12 +384,7 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
             if (gscore >= 0 && gscore < 1e100) atomicMin(&f.ctr->glitch_min_bits, (unsigned long long)__double_as_longlong(gscore));
         }
     }
-    atomicAdd(&f.ctr->steps, n_steps);
-    atomicAdd(&f.ctr->bla_applies, n_bla);
-    atomicAdd(&f.ctr->bla_skipped, n_skip);
-    atomicAdd(&f.ctr->effective_iters, n_eff);
-    atomicAdd(&f.ctr->interior, n_int);
-    atomicAdd(&f.ctr->finished, n_fin);
+    exact_counts(f.ctr, s_counts, n_steps, n_bla, n_skip, n_eff, n_int, n_fin, 32);
 }
 
 // ---------------------------------------------------------------------------
@@ -996,6 +1013,8 @@ __device__ __forceinline__ void fe_escape_value(const FeParams& p, PixOut& o) {
 
 template <int OC>
 __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
+    __shared__ BlockCounts s_counts;
+    block_counts_init(s_counts);
     if (p.lanes_per_warp && (int)(threadIdx.x & 31u) >= p.lanes_per_warp) return;
     const FrameGeom& g = p.g;
     unsigned long long n_steps = 0, n_bla = 0, n_skip = 0, n_eff = 0;
@@ -1038,12 +1057,7 @@ __global__ void __launch_bounds__(128) k_fe_pass(DeviceFrame f, FeParams p) {
             ++n_int;
         }
     }
-    atomicAdd(&f.ctr->steps, n_steps);
-    atomicAdd(&f.ctr->bla_applies, n_bla);
-    atomicAdd(&f.ctr->bla_skipped, n_skip);
-    atomicAdd(&f.ctr->effective_iters, n_eff);
-    atomicAdd(&f.ctr->interior, n_int);
-    atomicAdd(&f.ctr->finished, n_fin);
+    exact_counts(f.ctr, s_counts, n_steps, n_bla, n_skip, n_eff, n_int, n_fin, lanes);
 }
 
 // ---------------------------------------------------------------------------
@@ -1273,6 +1287,8 @@ __global__ void __launch_bounds__(512) k_direct(DeviceFrame f, ShallowParams p) 
     using Sample = DirectSample<FORM, DERIV, OC>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_live[16], s_stop;
+    __shared__ BlockCounts s_counts;
+    block_counts_init(s_counts);
     const FrameGeom& g = p.g;
     const int n_all = f.px.n;
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
@@ -1445,9 +1461,7 @@ __global__ void __launch_bounds__(512) k_direct(DeviceFrame f, ShallowParams p) 
             direct_write<FORM, OC>(f, p, reinterpret_cast<DirectDone*>(smem)[64 * (kBins * w + k) + at]);
         }
     }
-    atomicAdd(&f.ctr->effective_iters, n_eff);
-    atomicAdd(&f.ctr->steps, n_steps);
-    atomicAdd(&f.ctr->interior, n_int);
+    exact_counts(f.ctr, s_counts, n_steps, 0, 0, n_eff, n_int, 0, 32);
 }
 
 // ---------------------------------------------------------------------------

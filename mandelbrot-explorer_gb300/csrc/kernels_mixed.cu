@@ -15,6 +15,7 @@
 // are validated against the arbitrary-precision oracle, not bit-compared.
 #include <cuda_runtime.h>
 
+#include "counts.cuh"
 #include "engine.h"
 #include "mixed_lane.cuh"
 
@@ -131,6 +132,35 @@ __device__ bool stage_orbit(float2* smem, const float2* g, int entries, unsigned
     return mbar_wait_bounded(mb, 1 << 22);
 }
 
+__device__ __forceinline__ void lane_counts(Counters* c, BlockCounts& s, unsigned n_steps, unsigned n_bla, unsigned long long n_skip, unsigned long long n_eff, unsigned n_rebase, unsigned n_exact,
+                                            unsigned n_ferebase, unsigned n_fin, unsigned n_int, unsigned n_intflag, unsigned n_escflag) {
+    block_count(s, 0, n_steps);
+    block_count(s, 1, n_bla);
+    block_count(s, 2, n_skip);
+    block_count(s, 3, n_eff);
+    block_count(s, 4, n_rebase);
+    block_count(s, 5, n_exact);
+    block_count(s, 6, n_ferebase);
+    block_count(s, 7, n_fin);
+    block_count(s, 8, n_int);
+    block_count(s, 9, n_intflag);
+    block_count(s, 10, n_escflag);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        counts_flush(&c->steps, s.v[0]);
+        counts_flush(&c->bla_applies, s.v[1]);
+        counts_flush(&c->bla_skipped, s.v[2]);
+        counts_flush(&c->effective_iters, s.v[3]);
+        counts_flush(&c->rebases, s.v[4]);
+        counts_flush(&c->exact_steps, s.v[5]);
+        counts_flush(&c->fe_rebases, s.v[6]);
+        counts_flush(&c->finished, s.v[7]);
+        counts_flush(&c->interior, s.v[8]);
+        counts_flush(&c->interior_flagged, s.v[9]);
+        counts_flush(&c->escape_flagged, s.v[10]);
+    }
+}
+
 // Iterations a lane takes per lane_run call between the warp's refill points
 // (MixedParams::lane_budget, a tuning axis: the span of the orbit a warp walks
 // between refills). Longer calls amortise the warp's reconvergence and refill
@@ -160,6 +190,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_lane_pass(DeviceFrame f, MixedPa
     // Blocks past the work leave at once (the work counter hands all n entries
     // to the lower blocks), before any orbit staging.
     if ((long long)blockIdx.x * (MAXT / 32) * LANES >= n) return;
+    __shared__ BlockCounts s_counts;
+    block_counts_init(s_counts);
     const unsigned take = LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u);
     bool stage_late = false;
     if (LaneReal<T>::kTrackError && p.orbit_in_smem) {
@@ -263,17 +295,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_lane_pass(DeviceFrame f, MixedPa
             live = false;
         }
     }
-    atomicAdd(&f.ctr->steps, (unsigned long long)n_steps);
-    atomicAdd(&f.ctr->bla_applies, (unsigned long long)n_bla);
-    atomicAdd(&f.ctr->bla_skipped, n_skip);
-    atomicAdd(&f.ctr->effective_iters, n_eff);
-    atomicAdd(&f.ctr->rebases, (unsigned long long)n_rebase);
-    atomicAdd(&f.ctr->exact_steps, (unsigned long long)n_exact);
-    atomicAdd(&f.ctr->fe_rebases, (unsigned long long)n_ferebase);
-    atomicAdd(&f.ctr->finished, n_fin);
-    if (n_intflag) atomicAdd(&f.ctr->interior_flagged, n_intflag);
-    if (n_escflag) atomicAdd(&f.ctr->escape_flagged, n_escflag);
-    atomicAdd(&f.ctr->interior, n_int);
+    lane_counts(f.ctr, s_counts, n_steps, n_bla, n_skip, n_eff, n_rebase, n_exact, n_ferebase, n_fin, n_int, n_intflag, n_escflag);
     if (stage_late && !mbar_wait_bounded((unsigned)__cvta_generic_to_shared(&mbar), 1 << 24) && threadIdx.x == 0) atomicAdd(&f.ctr->stage_timeouts, 1u << 16);
 }
 
@@ -306,6 +328,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch_pass(BatchArgs a) {
     const unsigned n = a.queue ? min(*a.queue_n, a.capacity) : a.total;
     if (a.wide_from && (n >= a.wide_from) != (LANES == 32)) return;
     if ((unsigned long long)blockIdx.x * (MAXT / 32) * LANES >= n) return;
+    __shared__ BlockCounts s_counts;
+    block_counts_init(s_counts);
     const unsigned take = LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u);
     const unsigned lane_id = threadIdx.x & 31;
     // per-thread counts of one pass (32-bit: a thread executes far fewer than
@@ -412,15 +436,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch_pass(BatchArgs a) {
             live = false;
         }
     }
-    atomicAdd(&a.ctr->steps, (unsigned long long)n_steps);
-    atomicAdd(&a.ctr->bla_applies, (unsigned long long)n_bla);
-    atomicAdd(&a.ctr->bla_skipped, n_skip);
-    atomicAdd(&a.ctr->effective_iters, n_eff);
-    atomicAdd(&a.ctr->rebases, (unsigned long long)n_rebase);
-    atomicAdd(&a.ctr->exact_steps, (unsigned long long)n_exact);
-    atomicAdd(&a.ctr->fe_rebases, (unsigned long long)n_ferebase);
-    atomicAdd(&a.ctr->finished, n_fin);
-    atomicAdd(&a.ctr->interior, n_int);
+    lane_counts(a.ctr, s_counts, n_steps, n_bla, n_skip, n_eff, n_rebase, n_exact, n_ferebase, n_fin, n_int, 0, 0);
 }
 
 // Between the probe and the main pass: interior detection of each view follows
