@@ -161,12 +161,25 @@ __device__ __forceinline__ void lane_counts(Counters* c, BlockCounts& s, unsigne
     }
 }
 
-// Iterations a lane takes per lane_run call between the warp's refill points
-// (MixedParams::lane_budget, a tuning axis: the span of the orbit a warp walks
-// between refills). Longer calls amortise the warp's reconvergence and refill
-// (measured on the 1080p 1e-300 frame: FP32 passes 6.0 ms at 32, 5.4 at 128,
-// 4.6 at 256, 4.7 at 1024); finished lanes return at once and wait for the
-// warp's next refill. Where a call ends changes no result.
+// Iterations a lane takes per lane_run call between the warp's refill points:
+// the span of the orbit a warp walks between refills, lane_calls times the
+// tuning axis (MixedParams::lane_budget, 256). Finished lanes return at once
+// and wait for the warp's next refill. Where a call ends changes no result.
+// A call takes as long as its slowest lane, and iterations differ tenfold in
+// cost between a lane's stretches (BLA skips, fast runs, single steps), so
+// short calls wait for more of them. Passes over more than twice their resident
+// lanes walk kCalls budgets a call. FP32 / double-float passes at 256, 512,
+// 1024, 2048 and 4096 iterations a call: 24 tiles of 256x256 at 1e-500 127, 99,
+// 73, 54, 54 / 158, 133, 106, 82, 79 ms; 1080p minibrot at 1e-1000 34.8, 34.4,
+// 31.8, 30.8, 32.7 / 38, 38, 38, 28, 27 ms (with the probe's calls short: FP32
+// 28.4). A smaller pass waits for its longest samples, whose warps run
+// them faster when its lanes meet again often: 8 tiles of 96x96 2.6 ms at 256
+// and 4.4 at 2048 in the double-float pass, 8 of 128x128 (1.05 times the
+// resident lanes) 3.0 and 4.4; from 2.3 times on long calls won (16 of 128x128:
+// 10.2 -> 8.2 FP32, 11.2 -> 8.1).
+// A probe's calls are one lane_budget: all its lanes end with the first decision.
+constexpr int kCalls = 8;
+__device__ __forceinline__ int lane_calls(unsigned n, unsigned block_lanes) { return n > 2 * gridDim.x * block_lanes ? kCalls : 1; }
 
 // The lane pass, persistent: warps pull samples from the pass's work counter
 // and refill idle lanes together. T = float is the mixed pass (orbit staged in
@@ -223,7 +236,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_lane_pass(DeviceFrame f, MixedPa
     Lane<T> L;
     unsigned cost0 = 0;
     bool live = false, exhausted = false, stop = false;
-    unsigned rounds = 0;
+    const int calls = FASTI || p.probe_stop ? 1 : lane_calls((unsigned)n, MAXT / 32 * LANES);
+    unsigned rounds = 0; // calls of lane_budget since the last look at the cancel flag
     for (;;) {
         // Warp-synchronous refill: every idle lane takes a new sample together,
         // so the per-sample setup runs once for all of them.
@@ -257,7 +271,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_lane_pass(DeviceFrame f, MixedPa
         }
         if (live) {
             T zrad = T(0);
-            const int st = lane_run<T, INTR, FASTI, DE>(L, p.lane_budget, f, p, bt, orb, reflen, ESC2f, blamask, zrad, n_steps, n_bla, n_skip, n_rebase, n_exact, n_ferebase);
+            const int st = lane_run<T, INTR, FASTI, DE>(L, calls * p.lane_budget, f, p, bt, orb, reflen, ESC2f, blamask, zrad, n_steps, n_bla, n_skip, n_rebase, n_exact, n_ferebase);
             if (p.probe_stop && (st == 2 || st == 4)) atomicExch(&f.ctr->probe_hit, 1u);
             if (st != 0 && f.out.cost) f.out.cost[L.oidx] = (unsigned)(n_steps + 4 * n_bla) - cost0;
             if (st == 1) {
@@ -289,10 +303,14 @@ __global__ void __launch_bounds__(MAXT, MINB) k_lane_pass(DeviceFrame f, MixedPa
                 live = false;
             }
         }
-        if (((++rounds & 31u) == 0) && mcancelled(f)) {
-            stop = true;
-            exhausted = true;
-            live = false;
+        rounds += (unsigned)calls;
+        if (rounds >= 32) {
+            rounds = 0;
+            if (mcancelled(f)) {
+                stop = true;
+                exhausted = true;
+                live = false;
+            }
         }
     }
     lane_counts(f.ctr, s_counts, n_steps, n_bla, n_skip, n_eff, n_rebase, n_exact, n_ferebase, n_fin, n_int, n_intflag, n_escflag);
@@ -338,10 +356,11 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch_pass(BatchArgs a) {
     unsigned long long n_skip = 0, n_eff = 0;
     unsigned int n_int = 0, n_fin = 0;
     Lane<T> L;
+    const int calls = a.view_interior ? 1 : lane_calls(n, MAXT / 32 * LANES);
     int view = 0;
     unsigned cost0 = 0, bla0 = 0;
     bool live = false, exhausted = false, stop = false;
-    unsigned rounds = 0;
+    unsigned rounds = 0; // calls of lane_budget since the last look at the cancel flag
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, !live) & take;
         if (idle && !exhausted) {
@@ -395,7 +414,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch_pass(BatchArgs a) {
             const ViewDesc& vd = a.views[view];
             const BlaEntry<T>* bt = vd.f.bla.use ? ViewTables<T>::bla(vd) : nullptr;
             T zrad = T(0);
-            const int st = lane_run<T, true, false, DE>(L, vd.p.lane_budget, vd.f, vd.p, bt, ViewTables<T>::orb(vd), vd.p.mx_ref_it + 1, T(vd.p.esc2f), (1 << vd.f.bla.minlevel) - 1, zrad,
+            const int st = lane_run<T, true, false, DE>(L, calls * vd.p.lane_budget, vd.f, vd.p, bt, ViewTables<T>::orb(vd), vd.p.mx_ref_it + 1, T(vd.p.esc2f), (1 << vd.f.bla.minlevel) - 1, zrad,
                                                        n_steps, n_bla, n_skip, n_rebase, n_exact, n_ferebase);
             // the learned ordering's costs: the FP32 tier's (the rerun tiers keep them)
             if (std::is_same<T, float>::value && st != 0 && vd.f.out.cost) {
@@ -430,10 +449,14 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch_pass(BatchArgs a) {
                 live = false;
             }
         }
-        if (((++rounds & 31u) == 0) && a.cancel && *a.cancel) {
-            stop = true;
-            exhausted = true;
-            live = false;
+        rounds += (unsigned)calls;
+        if (rounds >= 32) {
+            rounds = 0;
+            if (a.cancel && *a.cancel) {
+                stop = true;
+                exhausted = true;
+                live = false;
+            }
         }
     }
     lane_counts(a.ctr, s_counts, n_steps, n_bla, n_skip, n_eff, n_rebase, n_exact, n_ferebase, n_fin, n_int, 0, 0);

@@ -1279,15 +1279,6 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
     const Z ESC2hi = ESC2z * R::kEscHi, ESC2lo = ESC2z * R::kEscLo;
     // DE colourings: the derivative J advances with the delta (DE lanes only)
     const bool deriv = DE && g.deriv;
-    // The double-float lane with interior detection runs its general code, where
-    // lanes at different places of the orbit execute different paths (7.5 of 32
-    // lanes to an instruction on the period-1331 minibrot frame). Its calls
-    // end at the wrap of a short period, so that a warp's lanes take each
-    // period's BLA skips together: double-float tier 43 -> 35.6 ms there. Not
-    // for a period longer than a call's entries (24 tiles, period 38045: 2 %
-    // slower), and not for the FP32 lane, whose lanes lose more by waiting (34
-    // -> 49 ms).
-    const bool sync = std::is_same<T, df32>::value && INTR && p.use_interior && per > 0 && per <= 16 * budget;
     for (int b = 0; b < budget; ++b) {
         if constexpr (std::is_same<T, float>::value && !FASTI) {
             if (!(INTR && p.use_interior) && p.Zq) {
@@ -1439,11 +1430,7 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                 L.m += skip;
                 L.iter += skip;
                 L.rm += skip;
-                bool wrapped = false;
-                if (per && L.rm >= per) {
-                    L.rm -= per;
-                    wrapped = sync;
-                }
+                if (per && L.rm >= per) L.rm -= per;
                 lane_refresh(L);
                 L.Xc = orb[L.rm];
                 if (R::kTrackError) {
@@ -1457,7 +1444,6 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                 L.period_win = 1;
                 L.conf_P = 0;
                 L.conf_giveup = 0;
-                if (wrapped) return 0;
                 continue;
             }
         }
@@ -1552,11 +1538,7 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
         ++L.m;
         ++L.iter;
         ++L.rm;
-        bool wrapped = false;
-        if (per && L.rm == per) {
-            L.rm = 0;
-            wrapped = sync;
-        }
+        if (per && L.rm == per) L.rm = 0;
         L.Xc = orb[L.rm];
         T zr, zi;
         if constexpr (std::is_same<T, df32>::value) {
@@ -1729,7 +1711,6 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
                 ++n_rebase;
             }
         }
-        if (wrapped) return 0;
     }
     return 0;
 }
