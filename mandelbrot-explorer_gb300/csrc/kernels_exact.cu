@@ -527,9 +527,9 @@ __device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int
                 else
                     return 0;
             } else {
-                double wmag = sqrt(wm2);
+                double wmag = int_sqrt(wm2);
                 S = fe_mul(S, fe_from(wmag));
-                double inv = 1.0 / wmag;
+                double inv = int_div(1.0, wmag);
                 wr = nwr * inv;
                 wi = nwi * inv;
             }
@@ -540,14 +540,14 @@ __device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int
             FE nzi = fe_add(fe_add(fe_mul_d(dzr, bc.y), fe_mul_d(dzi, bc.x)), fe_add(fe_mul_d(dcrfe, bc.w), fe_mul_d(dcife, bc.z)));
             double fr = zl.x + fe_to_double(nzr), fi = zl.y + fe_to_double(nzi);
             if (fr * fr + fi * fi > ESC2) return 0;
-            FE Snew = fe_sqrt(fe_add(fe_mul(nzr, nzr), fe_mul(nzi, nzi)));
+            FE Snew = fe_sqrt<true>(fe_add(fe_mul(nzr, nzr), fe_mul(nzi, nzi)));
             if (Snew.m == 0.0) {
                 S = fe_make(1.0, 0);
                 wr = wi = 0.0;
             } else {
                 S = Snew;
-                wr = fe_to_double(fe_div(nzr, S));
-                wi = fe_to_double(fe_div(nzi, S));
+                wr = fe_to_double(fe_div<true>(nzr, S));
+                wi = fe_to_double(fe_div<true>(nzi, S));
             }
         }
         if (ab) {
@@ -603,14 +603,14 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
     const int reflen = p.mx_ref_it + 1;
     const int per = p.per;
     int rm = 0;
-    FE S = fe_sqrt(fe_add(fe_mul(dcr, dcr), fe_mul(dci, dci)));
+    FE S = fe_sqrt<true>(fe_add(fe_mul(dcr, dcr), fe_mul(dci, dci)));
     double wr, wi, dr, di;
     if (d_is_zero(S.m)) {
         S = fe_make(1.0, 0);
         wr = wi = dr = di = 0.0;
     } else {
-        wr = fe_to_double(fe_div(dcr, S));
-        wi = fe_to_double(fe_div(dci, S));
+        wr = fe_to_double(fe_div<true>(dcr, S));
+        wi = fe_to_double(fe_div<true>(dci, S));
         dr = wr;
         di = wi;
     }
@@ -667,15 +667,15 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
                     FE Jr = fe_mul_d(SJ, jr), Ji = fe_mul_d(SJ, ji);
                     FE nJr = fe_add(fe_sub(fe_mul_d(Jr, ab[0]), fe_mul_d(Ji, ab[1])), fe_from(ab[2]));
                     FE nJi = fe_add(fe_add(fe_mul_d(Jr, ab[1]), fe_mul_d(Ji, ab[0])), fe_from(ab[3]));
-                    SJ = fe_sqrt(fe_add(fe_mul(nJr, nJr), fe_mul(nJi, nJi)));
+                    SJ = fe_sqrt<true>(fe_add(fe_mul(nJr, nJr), fe_mul(nJi, nJi)));
                     if (d_is_zero(SJ.m)) {
                         SJ = fe_make(1.0, 0);
                         jr = ji = 0.0;
                         invSJd = 1.0;
                     } else {
-                        jr = fe_to_double(fe_div(nJr, SJ));
-                        ji = fe_to_double(fe_div(nJi, SJ));
-                        invSJd = 1.0 / fe_to_double(SJ);
+                        jr = fe_to_double(fe_div<true>(nJr, SJ));
+                        ji = fe_to_double(fe_div<true>(nJi, SJ));
+                        invSJd = int_div(1.0, fe_to_double(SJ));
                     }
                 }
                 m += skip;
@@ -684,8 +684,8 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
                 if (per && rm >= per) rm -= per;
                 s = fe_to_double(S);
                 S2 = fe_mul(S, S);
-                dr = fe_to_double(fe_div(dcr, S));
-                di = fe_to_double(fe_div(dci, S));
+                dr = fe_to_double(fe_div<true>(dcr, S));
+                di = fe_to_double(fe_div<true>(dci, S));
                 swr = s * wr;
                 swi = s * wi;
                 zsr = 1e30;
@@ -724,8 +724,8 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
             fe_step_underflow(Xrfe, Xife, dcr, dci, S, wr, wi);
             s = fe_to_double(S);
             S2 = fe_mul(S, S);
-            dr = fe_to_double(fe_div(dcr, S));
-            di = fe_to_double(fe_div(dci, S));
+            dr = fe_to_double(fe_div<true>(dcr, S));
+            di = fe_to_double(fe_div<true>(dci, S));
         } else {
             wr = nwr;
             wi = nwi;
@@ -746,12 +746,12 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
                 double jm2 = 1.0;
                 if (hj < kFeWLo || hj >= kFeWHi) jm2 = jr * jr + ji * ji;
                 if (d_abs_less(1e16, jm2) || (d_abs_less(jm2, 1e-16) && !d_is_zero(jm2))) {
-                    FE jmag = fe_sqrt(fe_from(jm2));
+                    FE jmag = fe_sqrt<true>(fe_from(jm2));
                     SJ = fe_mul(SJ, jmag);
-                    double inv = 1.0 / fe_to_double(jmag);
+                    double inv = int_div(1.0, fe_to_double(jmag));
                     jr *= inv;
                     ji *= inv;
-                    invSJd = 1.0 / fe_to_double(SJ);
+                    invSJd = int_div(1.0, fe_to_double(SJ));
                 }
             }
         }
@@ -833,15 +833,15 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
         }
         // |w|^2 > 1e16, or 0 < |w|^2 < 1e-16 (|w|^2 >= +0 or NaN)
         if (d_abs_less(1e16, wmag2) || (d_abs_less(wmag2, 1e-16) && !d_is_zero(wmag2))) {
-            FE wmag = fe_sqrt(fe_from(wmag2));
+            FE wmag = fe_sqrt<true>(fe_from(wmag2));
             S = fe_mul(S, wmag);
             s = fe_to_double(S);
             S2 = fe_mul(S, S);
-            double inv = 1.0 / fe_to_double(wmag);
+            double inv = int_div(1.0, fe_to_double(wmag));
             wr *= inv;
             wi *= inv;
-            dr = fe_to_double(fe_div(dcr, S));
-            di = fe_to_double(fe_div(dci, S));
+            dr = fe_to_double(fe_div<true>(dcr, S));
+            di = fe_to_double(fe_div<true>(dci, S));
             keep = false;
         }
         double dzmag2 = s * s * (keep ? wmag2 : wr * wr + wi * wi);
@@ -853,17 +853,17 @@ __device__ PixOut pixel_fe(const DeviceFrame& f, const FeParams& p, FE dcr, FE d
             FE zradfe = fe_add(fe_mul(zrfe, zrfe), fe_mul(zife, zife));
             FE dzfe = fe_add(fe_mul(Swr, Swr), fe_mul(Swi, Swi));
             if ((!per && m >= reflen) || fe_abs_less(zradfe, dzfe)) {
-                FE Snew = fe_sqrt(zradfe);
+                FE Snew = fe_sqrt<true>(zradfe);
                 if (d_is_zero(Snew.m)) {
                     wr = wi = 0.0;
                 } else {
                     S = Snew;
                     s = fe_to_double(S);
                     S2 = fe_mul(S, S);
-                    wr = fe_to_double(fe_div(zrfe, S));
-                    wi = fe_to_double(fe_div(zife, S));
-                    dr = fe_to_double(fe_div(dcr, S));
-                    di = fe_to_double(fe_div(dci, S));
+                    wr = fe_to_double(fe_div<true>(zrfe, S));
+                    wi = fe_to_double(fe_div<true>(zife, S));
+                    dr = fe_to_double(fe_div<true>(dcr, S));
+                    di = fe_to_double(fe_div<true>(dci, S));
                 }
                 m = 0;
                 rm = -1;
