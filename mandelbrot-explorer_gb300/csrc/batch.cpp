@@ -323,6 +323,15 @@ int BatchRunner::run(const mbx_request* reqs, int n, mbx_stats* view_stats, mbx_
         }
         ~Threads() { join(); }
     } direct;
+    auto failed = [&]() -> int {
+        direct.join();
+        for (int i = 0; i < n; ++i)
+            if (rcs[(size_t)i] != MBX_OK) {
+                err = eng_[i]->error();
+                return rcs[(size_t)i];
+            }
+        return MBX_OK;
+    };
     {
         // The frames' host work (GMP reference orbits, nucleus searches) is
         // independent per engine: up to `lanes` engines build concurrently,
@@ -366,10 +375,7 @@ int BatchRunner::run(const mbx_request* reqs, int n, mbx_stats* view_stats, mbx_
         std::unique_lock<std::mutex> l(mu);
         cv.wait(l, [&] { return prepared == shared.size(); });
         for (int i : shared)
-            if (rcs[(size_t)i] != MBX_OK) {
-                err = eng_[i]->error();
-                return rcs[(size_t)i];
-            }
+            if (rcs[(size_t)i] != MBX_OK) return failed(); // (the first frame's that failed, own ones included)
     }
     std::vector<int> deferred;
     for (int i = 0; i < n; ++i)
@@ -565,12 +571,7 @@ int BatchRunner::run(const mbx_request* reqs, int n, mbx_stats* view_stats, mbx_
             }
         }
     }
-    direct.join();
-    for (int i = 0; i < n; ++i)
-        if (rcs[(size_t)i] != MBX_OK) {
-            err = eng_[i]->error();
-            return rcs[(size_t)i];
-        }
+    if (const int rc = failed()) return rc;
     if (view_stats)
         for (int i = 0; i < n; ++i) view_stats[i] = vst[i];
     if (batch_stats) *batch_stats = bs;
