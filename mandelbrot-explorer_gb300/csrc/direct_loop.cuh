@@ -272,14 +272,6 @@ struct DirectTrap {
             if (r < 1e30) circle_hi = (float)r * 1.000001f;
         }
     }
-    template <int OC>
-    MBX_HD void give(OrbitColor<OC>& oc) const {
-        if constexpr ((OC & kOcTrap) != 0) {
-            oc.trap.point2 = point2;
-            oc.trap.cross = bitsd(cross);
-            oc.trap.circle = circle;
-        }
-    }
 };
 
 } // namespace mbx
