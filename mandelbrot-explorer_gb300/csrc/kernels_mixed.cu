@@ -4,13 +4,13 @@
 // memory (staged once per block by a TMA bulk copy) or from L1/L2 when it does
 // not fit. On GB300 one FP64 instruction costs as much issue time as ~60 FP32
 // ones, so FP64 (and FP64-mantissa floatexp) is used only on rare events:
-//   * BLA skips: coefficients and validity radii come from the FP64 table;
-//     candidates are screened on integer exponents, decided and applied in FP64;
-//   * rebasing near |Z + dz| ~ |dz|: screened in FP32, decided in FP64-floatexp;
-//   * escape: screened in FP32 with a relative margin, decided and the smooth
-//     value computed from an FP64 reconstruction of z;
+//   * the BLA table's construction;
+//   * escape: screened with a relative margin, decided inside it on an FP64
+//     reconstruction of z; the distance values, once per sample;
 //   * interior detection: FP32 screen, FP64 at close returns and saves;
-//   * steps where the orbit is below FP32's range (exact floatexp step).
+//   * the double-float lane's rebase decisions that its screen leaves open.
+// BLA skips, rebases and steps below FP32's range run in the lane type with int
+// exponents.
 // Semantics follow the reference's rescaled loop (mp.cpp:3287-3618); results
 // are validated against the arbitrary-precision oracle, not bit-compared.
 #include <cuda_runtime.h>
@@ -184,9 +184,9 @@ __device__ __forceinline__ int lane_calls(unsigned n, unsigned block_lanes) { re
 // The lane pass, persistent: warps pull samples from the pass's work counter
 // and refill idle lanes together. T = float is the mixed pass (orbit staged in
 // shared memory when it fits; samples its error estimate cannot vouch for are
-// queued for the FP64 pass); T = double is that FP64 pass over the queue, whose
-// length it reads on the device.
-// LANES < 32: only the low LANES lanes of a warp take samples. The rerun
+// queued); T = df32 is the double-float pass over that queue, whose length it
+// reads on the device.
+// LANES < 32: only the low LANES lanes of a warp take samples. Short rerun
 // passes are latency-bound (few samples, long dependency chains), so spreading
 // their samples over more warps hides more latency than filling each warp.
 template <class T, int MAXT, int MINB, int LANES = 32, bool INTR = true, bool FASTI = false, bool DE = false>
@@ -663,8 +663,16 @@ cudaError_t Engine::run_df_pass(const DeviceFrame& f) {
     // the queue length is known only on the device: both widths are launched
     // and the one it selects runs
     p.wide_from = kWideLanesPerSm * (unsigned)nsm_;
-    auto narrow = p.g.deriv ? k_lane_pass<df32, 128, 3, 8, true, false, true> : k_lane_pass<df32, 128, 3, 8>;
-    auto wide = p.g.deriv ? k_lane_pass<df32, 128, 3, 32, true, false, true> : k_lane_pass<df32, 128, 3, 32>;
+    // Frames whose probe found no interior take the lane without interior
+    // detectors: with them the derivative's lane waits for instructions more
+    // than for anything else (3.1 of 7.4 warps per issue), and without them it
+    // fits four blocks an SM (1080p zoom frame 300 with distance
+    // estimation, 758M steps: pass 15.4 -> 13.7 ms; five blocks 13.2, but small frames lose up to
+    // 4 % on their longest samples to the spills).
+    auto narrow = p.g.deriv ? (p.use_interior ? k_lane_pass<df32, 128, 3, 8, true, false, true> : k_lane_pass<df32, 128, 3, 8, false, false, true>)
+                            : (p.use_interior ? k_lane_pass<df32, 128, 3, 8> : k_lane_pass<df32, 128, 3, 8, false>);
+    auto wide = p.g.deriv ? (p.use_interior ? k_lane_pass<df32, 128, 3, 32, true, false, true> : k_lane_pass<df32, 128, 4, 32, false, false, true>)
+                          : (p.use_interior ? k_lane_pass<df32, 128, 3, 32> : k_lane_pass<df32, 128, 4, 32, false>);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(narrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
