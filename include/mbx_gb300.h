@@ -141,7 +141,7 @@ typedef struct {
     int smem_orbit_limit;   /* stage the FP32 orbit into shared memory when it fits in this many bytes (0: never) */
     double rescale_window;  /* |w|^2 is kept in [1/window, window]; 1e4 to 1e16 */
     double pass_ms;         /* autotune: GPU time of the calibration pass with this shape */
-    int lane_budget;        /* iterations a lane walks per call between its warp's refill points (passes of many samples: eight times as many): 16 to 4096 */
+    int lane_budget;        /* iterations a lane walks per call between its warp's refill points (passes of many samples: 4 to 32 times as many): 16 to 4096 */
 } mbx_tuning;
 
 /* Sets the mixed-pass tuning of a context (values out of range are ignored). */
