@@ -367,9 +367,11 @@ int BatchRunner::run(const mbx_request* reqs, int n, mbx_stats* view_stats, mbx_
             for (size_t q = (size_t)t; q < own.size(); q += (size_t)own_lanes) rcs[(size_t)own[q]] = eng_[own[q]]->compute(reqs[own[q]], &vst[own[q]]);
             take_shared();
         };
-        for (int t = 0; t < own_lanes; ++t) direct.th.emplace_back(take_own, t);
+        // (without shared frames this thread is one of them)
+        for (int t = shared.empty() ? 1 : 0; t < own_lanes; ++t) direct.th.emplace_back(take_own, t);
         std::vector<std::thread> th;
         for (int t = 1; t < lanes - own_lanes; ++t) th.emplace_back(take_shared);
+        if (shared.empty() && own_lanes) take_own(0);
         take_shared();
         for (auto& x : th) x.join();
         std::unique_lock<std::mutex> l(mu);
