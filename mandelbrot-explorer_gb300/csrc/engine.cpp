@@ -38,7 +38,7 @@ inline FE mpf_fe(mpf_srcptr x) {
     if (mpf_sgn(x) == 0) return fe_make(0.0, 0);
     long ex;
     double d = mpf_get_d_2exp(&ex, x);
-    return fe_make(d, (int)ex);
+    return fe_make(d, (int64_t)ex);
 }
 // float_math.cpp:22-27.
 inline int exp_floor_log2(double x) {
@@ -217,7 +217,7 @@ FE FixedReal::to_fe() const { // bigfixed.h:305-320
     if (top < 0) return fe_make(0.0, 0);
     double mant = (double)limb[top] * 18446744073709551616.0 + (double)(top >= 1 ? limb[top - 1] : 0ull);
     FE r = fe_from(mant);
-    r.e += 64 * (top - L);
+    r.e += (int64_t)64 * (top - L);
     return sign < 0 ? fe_neg(r) : r;
 }
 

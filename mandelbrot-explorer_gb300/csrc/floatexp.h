@@ -137,20 +137,20 @@ MBX_HD double xldexp(double x, int k) {
     return xldexp_rare(x, k);
 }
 
-// m 2^e; the exponent is an int (|e| stays far below 2^31: a scale of 10^k needs
-// k decimal digits).
+// m 2^e. The exponent has 64 bits: a scale may be written 1e400000000, and |dz|^2
+// of its frame is below 2^-(2^31).
 struct FE {
     double m;
-    int e;
+    int64_t e;
 };
 
-MBX_HD FE fe_make(double m, int e) {
+MBX_HD FE fe_make(double m, int64_t e) {
     FE r;
     r.m = m;
     r.e = e;
     return r;
 }
-MBX_HD FE fe_renorm(double m, int e) {
+MBX_HD FE fe_renorm(double m, int64_t e) {
     const uint64_t b = dbits(m);
     if (d_normal(b)) return fe_make(bitsd((b & 0x800fffffffffffffull) | (1022ull << 52)), e + (int)((b >> 52) & 0x7ff) - 1022);
     if (d_is_zero(m)) return fe_make(0.0, 0);
@@ -162,11 +162,11 @@ MBX_COLD double fe_to_double_rare(FE a) {
     if (d_is_zero(a.m)) return 0.0;
     if (a.e > 1100) return bitsd(0x7ff0000000000000ull | (dbits(a.m) & 0x8000000000000000ull));
     if (a.e < -1100) return 0.0;
-    return xldexp(a.m, a.e);
+    return xldexp(a.m, (int)a.e);
 }
 MBX_HD double fe_to_double(FE a) {
     const uint64_t b = dbits(a.m);
-    if (d_normal(b) && (unsigned)((b >> 52) & 0x7ff) - 1u + (unsigned)a.e < 0x7feu) return bitsd(b + ((uint64_t)(int64_t)a.e << 52));
+    if (d_normal(b) && ((b >> 52) & 0x7ff) - 1u + (uint64_t)a.e < 0x7feu) return bitsd(b + ((uint64_t)a.e << 52));
     return fe_to_double_rare(a);
 }
 MBX_HD FE fe_mul(FE a, FE b) {
@@ -177,13 +177,14 @@ MBX_HD FE fe_mul_d(FE a, double b) {
     if (d_is_zero(a.m) || d_is_zero(b)) return fe_make(0.0, 0);
     return fe_renorm(a.m * b, a.e);
 }
-MBX_HD FE fe_scale2(FE a, int k) { return d_is_zero(a.m) ? a : fe_make(a.m, a.e + k); }
+MBX_HD FE fe_scale2(FE a, int64_t k) { return d_is_zero(a.m) ? a : fe_make(a.m, a.e + k); }
 MBX_HD FE fe_add(FE a, FE b) {
     if (d_is_zero(a.m)) return b;
     if (d_is_zero(b.m)) return a;
-    const int d = a.e - b.e;
-    if (d > 54) return a;
-    if (d < -54) return b;
+    const int64_t dw = a.e - b.e;
+    if (dw > 54) return a;
+    if (dw < -54) return b;
+    const int d = (int)dw;
     // the smaller exponent's mantissa aligned to the larger (one add for both orders)
     const bool first = d >= 0;
     const double big = first ? a.m : b.m, small = xldexp(first ? b.m : a.m, first ? -d : d);
@@ -285,7 +286,7 @@ MBX_HD double xsqrt(double x) {
 template <bool INT = false>
 MBX_HD FE fe_sqrt(FE a) {
     if (d_le_zero(a.m)) return fe_make(0.0, 0);
-    int e = a.e;
+    int64_t e = a.e;
     double m = a.m;
     if (e & 1) {
         m = d_twice(m);

@@ -404,9 +404,9 @@ __device__ void bla_rerescale_underflow(FE& S, double& wr, double& wi, double nw
 
 __device__ void fe_step_underflow(FE Xr, FE Xi, FE dcr, FE dci, FE& S, double& wr, double& wi) { // mp.cpp:2794-2835
     const double sm = S.m, sm2 = sm * sm;
-    const int se = S.e;
-    const int NONE = (int)0x80000000;
-    int e = NONE;
+    const int64_t se = S.e;
+    const int64_t NONE = (int64_t)0x8000000000000000ll;
+    int64_t e = NONE;
     const bool has_w = wr != 0.0 || wi != 0.0;
     if (has_w && Xr.m != 0.0) e = max(e, Xr.e + se);
     if (has_w && Xi.m != 0.0) e = max(e, Xi.e + se);
@@ -418,10 +418,10 @@ __device__ void fe_step_underflow(FE Xr, FE Xi, FE dcr, FE dci, FE& S, double& w
         wr = wi = 0.0;
         return;
     }
-    auto align = [e](double m, int te) -> double {
-        int d = te - e;
+    auto align = [e](double m, int64_t te) -> double {
+        int64_t d = te - e;
         if (m == 0.0 || d < -54) return 0.0;
-        return m * pow2i(d);
+        return m * pow2i((int)d);
     };
     const double xs_r = align(Xr.m * sm, Xr.e + se);
     const double xs_i = align(Xi.m * sm, Xi.e + se);
@@ -444,20 +444,20 @@ __device__ void fe_step_underflow(FE Xr, FE Xi, FE dcr, FE dci, FE& S, double& w
 
 __device__ void fe_deriv_underflow(FE zr, FE zi, FE& SJ, double& jr, double& ji, double& invSJd) { // mp.cpp:2842-2876
     double im = 0.5 / SJ.m;
-    int ie = 1 - SJ.e;
+    int64_t ie = 1 - SJ.e;
     if (im >= 1.0) {
         im *= 0.5;
         ++ie;
     }
     FE invSJ = fe_make(im, ie);
-    int e = invSJ.e;
+    int64_t e = invSJ.e;
     if (zr.m != 0.0) e = max(e, zr.e);
     if (zi.m != 0.0) e = max(e, zi.e);
     auto align = [e](FE x) -> double {
         if (x.m == 0.0) return 0.0;
-        int d = x.e - e;
+        int64_t d = x.e - e;
         if (d < -54) return 0.0;
-        return x.m * pow2i(d);
+        return x.m * pow2i((int)d);
     };
     double azr = align(zr), azi = align(zi);
     double ar = 2.0 * (azr * jr - azi * ji) + align(invSJ);
@@ -488,7 +488,7 @@ __device__ int bla_try_fe(const BlaView& b, const double2* Z, bool periodic, int
         // |w|^2 >= (the larger part)^2 >= 2^(2 k), k its binade, so |dz|^2's
         // exponent is at least S2.e + 2 k: above rmax2's, no radius holds
         const unsigned h = umax_(hi_abs(wr), hi_abs(wi));
-        const int lo = S2.e + 2 * ((int)(h >> 20) - 1023);
+        const int64_t lo = S2.e + 2 * ((int)(h >> 20) - 1023);
         if (h >= 0x20000000u && h < 0x5fe00000u && !d_is_zero(S2.m) && lo > rmax.e) return 0;
     }
     const FE dz2 = fe_mul(S2, fe_from(wr * wr + wi * wi));

@@ -149,7 +149,7 @@ MBX_HD TE<T> te_from_fe(FE a) {
     return te_norm((T)a.m, (int)a.e);
 }
 template <class T>
-MBX_HD FE fe_from_te(TE<T> a) { return a.m == T(0) ? fe_make(0.0, 0) : fe_make((double)a.m, a.e); }
+MBX_HD FE fe_from_te(TE<T> a) { return a.m == T(0) ? fe_make(0.0, 0) : fe_make((double)a.m, (int64_t)a.e); }
 
 // Per-type constants of the lane.
 template <class T>
@@ -695,8 +695,8 @@ MBX_RARE JVal lane_j_step_fe(FE Xr, FE Xi, FE S, double wr, double wi, int sje, 
     const FE sj = fe_make(0.5, sje), Jr = fe_mul_d(sj, jr), Ji = fe_mul_d(sj, ji);
     const FE nr = fe_add(fe_scale2(fe_sub(fe_mul(zr, Jr), fe_mul(zi, Ji)), 1), fe_make(0.5, 1));
     const FE ni = fe_scale2(fe_add(fe_mul(zr, Ji), fe_mul(zi, Jr)), 1);
-    const int e = d_is_zero(nr.m) ? ni.e : (d_is_zero(ni.m) ? nr.e : imax(nr.e, ni.e));
-    return JVal{fe_to_double(fe_make(nr.m, nr.e - e)), fe_to_double(fe_make(ni.m, ni.e - e)), e};
+    const int64_t e = d_is_zero(nr.m) ? ni.e : (d_is_zero(ni.m) ? nr.e : (nr.e > ni.e ? nr.e : ni.e));
+    return JVal{fe_to_double(fe_make(nr.m, nr.e - e)), fe_to_double(fe_make(ni.m, ni.e - e)), (int)e};
 }
 // J' = A J + B through a BLA skip, in pairs of floats for both lane types (the
 // FP32 lane rounds the result to float once; FP64 floatexp, as it was formed
