@@ -545,11 +545,6 @@ struct Lane {
     T jr, ji, invSJ, ezr, ezi;
 };
 
-// 2 x, exactly (of a double-float: both parts; what the product with 2 gives)
-MBX_HD float lane_twice(float x) { return x + x; }
-MBX_HD double lane_twice(double x) { return x + x; }
-MBX_HD df32 lane_twice(df32 x) { return df32(x.hi + x.hi, x.lo + x.lo); }
-
 // d = dc / S in units of S.
 template <class T>
 MBX_HD typename LaneReal<T>::V2 lane_d(T Sm, int k, typename LaneReal<T>::V2 dcm) {
@@ -642,19 +637,11 @@ MBX_HD void lane_j_window(Lane<T>& L) {
     lane_j_inv(L);
 }
 
-// J' = 2 z J + 1 with z at unit scale in the lane type.
-template <class T>
-MBX_HD void lane_j_step(Lane<T>& L, T zr, T zi) {
-    if constexpr (std::is_same<T, df32>::value) {
-        const cdf j = cd_twice(cd_cmul(zr, zi, cd_make(L.jr, L.ji)));
-        L.jr = cd_re(j) + L.invSJ;
-        L.ji = cd_im(j);
-    } else {
-        const T a = lane_twice(zr * L.jr - zi * L.ji) + L.invSJ;
-        const T b = lane_twice(zr * L.ji + zi * L.jr);
-        L.jr = a;
-        L.ji = b;
-    }
+// J' = 2 z J + 1 with z at unit scale, in the double-float lane.
+MBX_HD void lane_j_step(Lane<df32>& L, df32 zr, df32 zi) {
+    const cdf j = cd_twice(cd_cmul(zr, zi, cd_make(L.jr, L.ji)));
+    L.jr = cd_re(j) + L.invSJ;
+    L.ji = cd_im(j);
     lane_j_window(L);
 }
 // The FP32 lane's form, from 2 z = 2 X + 2 s w as the common-step loop forms it.
@@ -730,13 +717,8 @@ MBX_RARE JBla<T> lane_j_bla_df(T Ar, T Ai, int ea, T Br, T Bi, int eb, T Jr, T J
 }
 template <class T>
 MBX_HD void lane_j_bla(Lane<T>& L, const BlaEntry<T>& e) {
-    if constexpr (std::is_same<T, double>::value) {
-        const int E1 = e.ea + L.SJ.e - 1, E = imax(E1, e.eb);
-        lane_j_set(L, ldexp_ftz(e.ar * L.jr - e.ai * L.ji, E1 - E) + ldexp_ftz(e.br, e.eb - E), ldexp_ftz(e.ar * L.ji + e.ai * L.jr, E1 - E) + ldexp_ftz(e.bi, e.eb - E), E);
-    } else {
-        const JBla<T> v = lane_j_bla_df<T>(e.ar, e.ai, e.ea, e.br, e.bi, e.eb, L.jr, L.ji, L.SJ.e - 1);
-        lane_j_set(L, v.r, v.i, v.e);
-    }
+    const JBla<T> v = lane_j_bla_df<T>(e.ar, e.ai, e.ea, e.br, e.bi, e.eb, L.jr, L.ji, L.SJ.e - 1);
+    lane_j_set(L, v.r, v.i, v.e);
 }
 // dz = S w with S <- |v| 2^e and w <- v / |v| for a vector v scaled by 2^e.
 template <class T>
@@ -849,15 +831,7 @@ MBX_HD void lane_z_double(const Lane<T>& L, const double2* Zd, double& zr, doubl
 // variance added, the existing error carried by g2 = |2 z|^2).
 template <class T>
 MBX_HD void lane_step(typename LaneReal<T>::V2 X, T s, T wr, T wi, T dr, T di, typename LaneReal<T>::E err2, typename LaneReal<T>::E g2, T& nwr, T& nwi,
-                      typename LaneReal<T>::E& nerr2) {
-    using R = LaneReal<T>;
-    const T fR = lane_twice(X.x) + s * wr;
-    const T fI = lane_twice(X.y) + s * wi;
-    nwr = fR * wr - fI * wi + dr;
-    nwi = fR * wi + fI * wr + di;
-    const typename R::E a = R::toe(nwr), c = R::toe(nwi);
-    nerr2 = err2 * g2 + R::kEps2 * (a * a + c * c);
-}
+                      typename LaneReal<T>::E& nerr2);
 
 // The FP32 step with its operations spelled out: f = 2 X + s w as one paired
 // FMA (f32x2), w' = f w + d as four FMAs, |w'|^2 and the error update as
@@ -877,7 +851,7 @@ MBX_HD void lane_step<float>(float2 X, float s, float wr, float wi, float dr, fl
     nerr2 = fmaf(err2, g2, LaneReal<float>::kEps2 * wm2);
 }
 
-// The double-float step in paired operations (the generic form's, part by part).
+// The double-float step in paired operations.
 template <>
 MBX_HD void lane_step<df32>(df2 X, df32 s, df32 wr, df32 wi, df32 dr, df32 di, float err2, float g2, df32& nwr, df32& nwi, float& nerr2) {
     const cdf w = cd_make(wr, wi), f = cd_twice(cd_make(X.x, X.y)) + cd_scale(s, w);
