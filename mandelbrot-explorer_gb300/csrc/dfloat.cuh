@@ -87,9 +87,13 @@ MBX_HD bool operator!=(df32 a, df32 b) { return !(a == b); }
 // Complex double-floats, real and imaginary part side by side: Blackwell's paired
 // FP32 instructions take both parts' operations at once. Each part goes through
 // the operations of operator+ and operator* above in their order (a difference
-// a - b as fma(b, -1, a), one rounding), so the bits are those of the scalar
-// forms; half the instructions matter because the lanes that use them wait for
-// instruction fetch.
+// a - b as fma(b, -1, a), one rounding). The unit that uses them is compiled with
+// contraction, which fuses products into sums of the scalar forms and leaves the
+// paired ones as they are written: their last bits can differ, about one value of
+// a frame in a hundred moved by a bit, and errors against the exact form stayed
+// the same (mean, 99 % and largest over some 30 outputs of zoom, minibrot, 1e-300
+// frames and tiles: ratios of 1.000). Half the instructions matter because the
+// lanes that use them wait for instruction fetch.
 struct cdf {
     float2 hi, lo;
 };

@@ -4,8 +4,11 @@
 // Semantics follow the reference's src/engine/floatexp.h:17-107 operation by
 // operation; frexp/ldexp are implemented on the IEEE bit patterns so that host
 // and device produce identical bits (ldexp rounds to nearest-even in the
-// subnormal range exactly like libm's). Everything here must be compiled
-// without FMA contraction (-ffp-contract=off / -fmad=false).
+// subnormal range exactly like libm's). The exact form and the host compile it
+// without FMA contraction (-ffp-contract=off / -fmad=false): there every
+// operation's bits are part of the result. The lane passes compile it with
+// contraction; the floatexp operations have no product that a sum could take in
+// but exact ones (by powers of two), so theirs are the same.
 #pragma once
 #include <stdint.h>
 #include <string.h>
@@ -200,9 +203,9 @@ MBX_HD FE fe_sub(FE a, FE b) { return fe_add(a, fe_neg(b)); }
 // 30-bit reciprocal (of b, of sqrt(x)) from a single-precision seed and one Newton
 // step, a first digit of 30 bits, the exact remainder modulo 2^64 (its magnitude
 // stays below 2^57), a second of 23 bits, and the rounding decided by the last
-// remainder. The exact loop takes them (its pass over the 1,330 leftovers of the
-// 1080p minibrot frame 24.6 -> 22.0 ms, over the 1080p frame at 1e-300 42.0 ->
-// 39.7); the lanes' called functions keep the plain operations (with these the
+// remainder. The exact loop takes them (its pass over the 1,276 leftovers of the
+// 1080p minibrot frame 24.5 -> 22.5 ms, over the 1080p frame at 1e-300 41.9 ->
+// 39.8); the lanes' called functions keep the plain operations (with these the
 // 1080p zoom frame took 24.7 ms instead of 23.4: more instructions to fetch).
 MBX_COLD double div_rare(double a, double b) { return a / b; }
 MBX_HD double int_div(double a, double b) {

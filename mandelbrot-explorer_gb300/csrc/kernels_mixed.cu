@@ -168,22 +168,27 @@ __device__ __forceinline__ void lane_counts(Counters* c, BlockCounts& s, unsigne
 // A call takes as long as its slowest lane, and iterations differ tenfold in
 // cost between a lane's stretches (BLA skips, fast runs, single steps), so
 // short calls wait for more of them. Passes over more than twice their resident
-// lanes walk kCalls budgets a call. FP32 / double-float passes at 256, 512,
-// 1024, 2048 and 4096 iterations a call: 24 tiles of 256x256 at 1e-500 127, 99,
-// 73, 54, 54 / 158, 133, 106, 82, 79 ms; 1080p minibrot at 1e-1000 34.8, 34.4,
-// 31.8, 30.8, 32.7 / 38, 38, 38, 28, 27 ms (with the probe's calls short: FP32
-// 28.4). A smaller pass waits for its longest samples, whose warps run
-// them faster when its lanes meet again often: 8 tiles of 96x96 2.6 ms at 256
-// and 4.4 at 2048 in the double-float pass, 8 of 128x128 (1.05 times the
-// resident lanes) 3.0 and 4.4; from 2.3 times on long calls won (16 of 128x128:
-// 10.2 -> 8.2 FP32, 11.2 -> 8.1).
+// lanes walk kCalls budgets a call. Double-float pass at 1, 2, 4, 8, 16 and 32
+// budgets of 256: 24 seed-drawn tiles of 256x256 at 1e-500 121, 94, 78, 62, 62, 61
+// ms (another seed 192, 157, 130, 106, 106, 103); 1080p minibrot at 1e-1000 38.6,
+// 36.7, 37.5, 27.7, 27.6, 27.9, its FP32 pass 33.1, 30.6, 30.4, 27.7, 26.9, 25.3.
+// A smaller pass waits for its longest samples, whose warps run them faster when
+// its lanes meet again often: double-float pass, one budget against eight, 8 tiles
+// of 64x64 4.9 and 6.9 ms, of 96x96 6.0 and 7.9, of 128x128 14.7 and 16.0, 16 of
+// them 19.1 and 19.3, 24 20.8 and 20.5.
 // A probe's calls are one lane_budget: all its lanes end with the first decision.
 constexpr int kCalls = 8;
-// The FP32 pass of a batch: where the learned order puts alike samples side by
-// side, its lanes wait least, and the longest calls are best (24 tiles: 33.4 ms
-// at 8 budgets, 32.1 at 32). In the natural order 4: 5 would take 40.5 ms and 8
-// 37.9 instead of 50.7 (80.3 at 1), but then the learned order gains less than
-// the fifth of the natural order's pass that its test holds it to.
+// The FP32 pass of a batch, ms at 1, 2, 4, 8, 16 and 32 budgets:
+//   natural order    24 tiles, seed 4:  82.7  65.1  51.5  38.1  37.8  37.5
+//                    24 tiles, seed 1: 127.3  99.7  74.0  54.0  53.0  52.2
+//                    64 tiles:         155.3 125.1  97.1  72.9  72.4  72.0
+//                    8 tiles:           27.9  25.3  21.5  17.3  16.7  17.1
+//   by probe cost, at 4, 8, 16, 32: 24 tiles, seed 4 40.1 33.4 33.3 32.7, seed 1
+//   47.9 38.5 37.4 36.0, 64 tiles 88.4 69.7 68.7 68.1, 8 tiles 19.3 16.7 16.3 16.0
+// In an order that puts alike samples side by side the lanes wait least, and the
+// longest calls are best. The natural order takes 4, and would be a quarter faster
+// at 8: there the trained order is 12 to 14 % faster than it, where its test asks
+// for a fifth, which it was when calls had one budget.
 constexpr int kCallsOrdered = 32, kCallsNatural = 4;
 __device__ __forceinline__ int lane_calls(unsigned n, unsigned block_lanes, int calls = kCalls) { return n > 2 * gridDim.x * block_lanes ? calls : 1; }
 

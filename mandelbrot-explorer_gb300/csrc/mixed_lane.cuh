@@ -688,7 +688,11 @@ MBX_RARE JVal lane_j_step_fe(FE Xr, FE Xi, FE S, double wr, double wi, int sje, 
 // J' = A J + B through a BLA skip, in pairs of floats for both lane types (the
 // FP32 lane rounds the result to float once; FP64 floatexp, as it was formed
 // before, took some 60 FP64 instructions of 64 cycles a skip and kept the FP32
-// pass's FP64 unit 60 % busy on a 1080p zoom frame).
+// pass's FP64 unit 60 % busy on a 1080p zoom frame). The pairs' 46 bits against
+// FP64's 53 are lost in the rounding to what the lane keeps: with the skip formed
+// in FP64 floatexp, all else as it is, 73 frames of the zoom, at 1e-300 and at the
+// minibrot (480x270; distances, angles, counts) and 8 tiles have the same bits in
+// all of 23.2 million values.
 template <class T>
 struct JBla {
     T r, i;

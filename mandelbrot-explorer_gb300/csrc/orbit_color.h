@@ -55,8 +55,9 @@ MBX_OC_HD double oc_double(unsigned long long b) {
 
 // sin(7 arg z) as Im(z^7) / |z|^7: z scaled to [1, 2) by its larger part's binade,
 // four complex products and a reciprocal square root, about 40 FP64 operations
-// where atan2 and sin take over 150. Its error is below theirs (2.5e-15 against
-// 4e-15: theirs begins with the rounding of 7 arg z). For a larger part in
+// where atan2 and sin take over 150. Its error is below theirs (on the device at
+// most 1.2e-15 against 4.5e-15 over 2.1e6 points in quadruple precision, 1.8e-16
+// against 4.7e-16 in the mean: theirs begins with the rounding of 7 arg z). For a larger part in
 // [2^-900, 2^900]; the plain form otherwise.
 MBX_OC_HD double stripe_sin7(double zr, double zi) {
     const double ar = fabs(zr), ai = fabs(zi), m = ar > ai ? ar : ai;

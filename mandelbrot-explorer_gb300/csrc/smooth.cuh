@@ -3,8 +3,8 @@
 // 90 and 60 FP64 instructions on GB300, whose FP64 unit takes one warp
 // instruction per 64 cycles. In pairs of floats (color_math.cuh) the logarithms
 // come within 2^-42, which settles the rounding to float on all but about one
-// value in 2^17; those take the double expression. So the values are the same
-// floats. Host and device; compiled without FMA contraction.
+// smooth count in 2^17 and one distance in 2^15 (whose window is taken wider);
+// those take the double expression. So the values are the same floats. Host and device; compiled without FMA contraction.
 #pragma once
 #include "color_math.cuh"
 #include "floatexp.h"
