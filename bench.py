@@ -677,7 +677,7 @@ def main():
                          "all_passes": {"achieved": achieved_all, "frac": achieved_all / fp32_peak if fp32_peak else None, "note": "every delta pass of the frames (FP32, double-float and exact-form tiers) over their GPU time"},
                          "peak_source": "measured in-run FMA issue rate (mbx_measure_fma_peak); MEASURED_PEAKS.json holds only HBM and bf16", "fp64_peak": fp64_peak,
                          "step_time_by_tier": tier_share,
-                         "note_largest": "by device time the double-float tier (k_lane_pass<df32>) is the step's largest kernel, on the minibrot frame: latency-bound chains of the longest samples (profiles/k_lane_pass_df32_minibrot1000_1080p_ncu.md), far below any throughput roof; the FP32 lane is reported as the roofline kernel because it carries the step's arithmetic"},
+                         "note_largest": "by device time the FP32 lanes and the double-float tier (k_lane_pass<df32>) take about a third of the step each, most of it on the minibrot frame: divergence and the longest samples' chains (profiles/k_lane_pass_minibrot1000_1080p_ncu.md), far below any throughput roof; the FP32 lane is reported as the roofline kernel because it carries the step's arithmetic"},
             "cpu_baseline": cpu,
             "clocks": clk,
             "gpu_launches": tot[3],
