@@ -105,6 +105,11 @@ __host__ __device__ inline void entry_coords(const PixelSet& px, int i, int* a) 
     a[3] = 0;
 }
 
+// The pass entry of a lane when a warp's 32 entries are four groups of eight
+// neighbours, one from each quarter of the set (a ticket is a warp's turn, tickets
+// = ceil(n / 32)): every entry below 32 * tickets once.
+__host__ __device__ inline int spread_entry(int ticket, int lane, int tickets) { return ((lane >> 3) * tickets + ticket) * 8 + (lane & 7); }
+
 struct Outputs {
     float* iter;     // (W*sub) x (H*sub), reference layout (getIndex mp.cpp:4334-4340)
     float* normal;   // DE overlay, may be null
@@ -162,6 +167,7 @@ struct Fp64Params {
     int use_interior, int_rep, interior_confirm;
     double interior_eps2;
     unsigned esc_word = 0;   // direct_escape_word(g.ESC2), set by launch_fp64_pass
+    int spread_tickets = 0;  // passes of at most this many warp turns take spread_entry's order
 };
 
 // Floatexp rescaled loop parameters (mp.cpp:3287-3618, 3620-3816).

@@ -133,12 +133,14 @@ __global__ void __launch_bounds__(128) k_fp64_pass(DeviceFrame f, Fp64Params p) 
     const double2* D = f.orbit.D;
     const CDivBy by_delta = c_div_by(p.sa_delta);
     const int bla_mask = (1 << f.bla.minlevel) - 1;
+    const int tickets = (int)(((unsigned)f.px.n + 31u) >> 5);
+    const bool spread = tickets <= p.spread_tickets;
     unsigned long long n_steps = 0, n_bla = 0, n_skip = 0, n_eff = 0;
     unsigned int n_int = 0, n_fin = 0;
     for (;;) {
         const int first = warp_take(f, f.px.n, 32);
         if (first < 0) break;
-        const int i = first + (int)(threadIdx.x & 31u);
+        const int i = spread ? spread_entry(first >> 5, (int)(threadIdx.x & 31u), tickets) : first + (int)(threadIdx.x & 31u);
         if (i >= f.px.n) continue;
         int arr[4];
         entry_key(f.px, i, arr);
