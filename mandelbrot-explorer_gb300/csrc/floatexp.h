@@ -141,60 +141,75 @@ MBX_HD double xldexp(double x, int k) {
 }
 
 // m 2^e. The exponent has 64 bits: a scale may be written 1e400000000, and |dz|^2
-// of its frame is below 2^-(2^31).
-struct FE {
+// of its frame is below 2^-(2^31). FEt<int> is for operands whose exponents are known
+// to leave an int's range nowhere.
+template <class E>
+struct FEt {
     double m;
-    int64_t e;
+    E e;
 };
+using FE = FEt<int64_t>;
 
-MBX_HD FE fe_make(double m, int64_t e) {
-    FE r;
+template <class E>
+MBX_HD FEt<E> fe_make_as(double m, E e) {
+    FEt<E> r;
     r.m = m;
     r.e = e;
     return r;
 }
-MBX_HD FE fe_renorm(double m, int64_t e) {
+MBX_HD FE fe_make(double m, int64_t e) { return fe_make_as<int64_t>(m, e); }
+template <class E>
+MBX_HD FEt<E> fe_renorm_as(double m, E e) {
     const uint64_t b = dbits(m);
-    if (d_normal(b)) return fe_make(bitsd((b & 0x800fffffffffffffull) | (1022ull << 52)), e + (int)((b >> 52) & 0x7ff) - 1022);
-    if (d_is_zero(m)) return fe_make(0.0, 0);
+    if (d_normal(b)) return fe_make_as<E>(bitsd((b & 0x800fffffffffffffull) | (1022ull << 52)), e + (int)((b >> 52) & 0x7ff) - 1022);
+    if (d_is_zero(m)) return fe_make_as<E>(0.0, 0);
     const FrexpOf r = xfrexp_rare(m);
-    return fe_make(r.m, e + r.e);
+    return fe_make_as<E>(r.m, e + r.e);
 }
+MBX_HD FE fe_renorm(double m, int64_t e) { return fe_renorm_as<int64_t>(m, e); }
 MBX_HD FE fe_from(double x) { return fe_renorm(x, 0); }
-MBX_COLD double fe_to_double_rare(FE a) {
+template <class E>
+MBX_COLD double fe_to_double_rare(FEt<E> a) {
     if (d_is_zero(a.m)) return 0.0;
     if (a.e > 1100) return bitsd(0x7ff0000000000000ull | (dbits(a.m) & 0x8000000000000000ull));
     if (a.e < -1100) return 0.0;
     return xldexp(a.m, (int)a.e);
 }
-MBX_HD double fe_to_double(FE a) {
+template <class E>
+MBX_HD double fe_to_double(FEt<E> a) {
     const uint64_t b = dbits(a.m);
-    if (d_normal(b) && ((b >> 52) & 0x7ff) - 1u + (uint64_t)a.e < 0x7feu) return bitsd(b + ((uint64_t)a.e << 52));
+    if (d_normal(b) && ((b >> 52) & 0x7ff) - 1u + (uint64_t)(int64_t)a.e < 0x7feu) return bitsd(b + ((uint64_t)(int64_t)a.e << 52));
     return fe_to_double_rare(a);
 }
-MBX_HD FE fe_mul(FE a, FE b) {
-    if (d_is_zero(a.m) || d_is_zero(b.m)) return fe_make(0.0, 0);
-    return fe_renorm(a.m * b.m, a.e + b.e);
+template <class E>
+MBX_HD FEt<E> fe_mul(FEt<E> a, FEt<E> b) {
+    if (d_is_zero(a.m) || d_is_zero(b.m)) return fe_make_as<E>(0.0, 0);
+    return fe_renorm_as<E>(a.m * b.m, a.e + b.e);
 }
-MBX_HD FE fe_mul_d(FE a, double b) {
-    if (d_is_zero(a.m) || d_is_zero(b)) return fe_make(0.0, 0);
-    return fe_renorm(a.m * b, a.e);
+template <class E>
+MBX_HD FEt<E> fe_mul_d(FEt<E> a, double b) {
+    if (d_is_zero(a.m) || d_is_zero(b)) return fe_make_as<E>(0.0, 0);
+    return fe_renorm_as<E>(a.m * b, a.e);
 }
-MBX_HD FE fe_scale2(FE a, int64_t k) { return d_is_zero(a.m) ? a : fe_make(a.m, a.e + k); }
-MBX_HD FE fe_add(FE a, FE b) {
+template <class E>
+MBX_HD FEt<E> fe_scale2(FEt<E> a, int64_t k) { return d_is_zero(a.m) ? a : fe_make_as<E>(a.m, a.e + (E)k); }
+template <class E>
+MBX_HD FEt<E> fe_add(FEt<E> a, FEt<E> b) {
     if (d_is_zero(a.m)) return b;
     if (d_is_zero(b.m)) return a;
-    const int64_t dw = a.e - b.e;
+    const E dw = a.e - b.e;
     if (dw > 54) return a;
     if (dw < -54) return b;
     const int d = (int)dw;
     // the smaller exponent's mantissa aligned to the larger (one add for both orders)
     const bool first = d >= 0;
     const double big = first ? a.m : b.m, small = xldexp(first ? b.m : a.m, first ? -d : d);
-    return fe_renorm(big + small, first ? a.e : b.e);
+    return fe_renorm_as<E>(big + small, first ? a.e : b.e);
 }
-MBX_HD FE fe_neg(FE a) { return fe_make(-a.m, a.e); }
-MBX_HD FE fe_sub(FE a, FE b) { return fe_add(a, fe_neg(b)); }
+template <class E>
+MBX_HD FEt<E> fe_neg(FEt<E> a) { return fe_make_as<E>(-a.m, a.e); }
+template <class E>
+MBX_HD FEt<E> fe_sub(FEt<E> a, FEt<E> b) { return fe_add(a, fe_neg(b)); }
 // Quotient and square root on integers, correctly rounded, for normal operands
 // and results. An FP64 division is some 9 FP64 instructions and a square root 10,
 // each of which holds its SM quarter's FP64 unit for 64 cycles; a BLA skip of the
@@ -268,12 +283,13 @@ MBX_HD double int_sqrt(double x) {
     q -= r2 <= -(int64_t)q ? 1 : 0;
     return bitsd(((uint64_t)((e - odd) / 2 + 1023) << 52) + (q - kOne));
 }
-template <bool INT = false>
-MBX_HD FE fe_div(FE a, FE b) {
-    if (d_is_zero(a.m)) return fe_make(0.0, 0);
-    return fe_renorm(INT ? int_div(a.m, b.m) : a.m / b.m, a.e - b.e);
+template <bool INT = false, class E>
+MBX_HD FEt<E> fe_div(FEt<E> a, FEt<E> b) {
+    if (d_is_zero(a.m)) return fe_make_as<E>(0.0, 0);
+    return fe_renorm_as<E>(INT ? int_div(a.m, b.m) : a.m / b.m, a.e - b.e);
 }
-MBX_HD bool fe_abs_less(FE a, FE b) {
+template <class E>
+MBX_HD bool fe_abs_less(FEt<E> a, FEt<E> b) {
     if (d_is_zero(a.m)) return !d_is_zero(b.m);
     if (d_is_zero(b.m)) return false;
     if (a.e != b.e) return a.e < b.e;
@@ -286,16 +302,16 @@ MBX_HD double xsqrt(double x) {
     return __builtin_sqrt(x);
 #endif
 }
-template <bool INT = false>
-MBX_HD FE fe_sqrt(FE a) {
-    if (d_le_zero(a.m)) return fe_make(0.0, 0);
-    int64_t e = a.e;
+template <bool INT = false, class E>
+MBX_HD FEt<E> fe_sqrt(FEt<E> a) {
+    if (d_le_zero(a.m)) return fe_make_as<E>(0.0, 0);
+    E e = a.e;
     double m = a.m;
     if (e & 1) {
         m = d_twice(m);
         --e;
     }
-    return fe_renorm(INT ? int_sqrt(m) : xsqrt(m), e / 2);
+    return fe_renorm_as<E>(INT ? int_sqrt(m) : xsqrt(m), e / 2);
 }
 
 // Complex arithmetic as GCC evaluates std::complex<double> for finite operands

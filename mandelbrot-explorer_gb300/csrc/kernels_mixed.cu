@@ -708,7 +708,7 @@ cudaError_t launch_batch_pass(int tier, const BatchArgs& a, int nsm, cudaStream_
             k_batch_pass<df32, 128, 3, 32, true><<<nsm * 4, 128, 0, st>>>(b);
         } else {
             // A long queue holds many waves of samples: four blocks of 128 per
-            // SM, at 128 registers with 70 bytes spilled around called functions
+            // SM, at 128 registers with 98 bytes spilled around called functions
             // (24 tiles of the 1e-500 image, 1.2M queued: 222 ms against 250 with
             // three). A short one waits for its longest sample: three, without the
             // spills (8 zoom frames of 64x36, 191 queued: 0.88 -> 0.81 ms, of

@@ -148,6 +148,12 @@ MBX_HD TE<T> te_from_fe(FE a) {
     if (a.m == 0.0) return TE<T>{T(0), 0};
     return te_norm((T)a.m, (int)a.e);
 }
+// An exponent whose floatexp operations (sums of two or three at most) an int
+// holds: with 64-bit ones in the rare steps the double-float pass of the 1080p
+// minibrot frame takes 27.7 ms instead of 26.3, of 24 tiles 104 instead of 102.
+MBX_HD bool te_mid(int64_t e) { return (uint64_t)(e + (1 << 28)) < (1u << 29); }
+template <class T>
+MBX_HD TE<double> te_double(TE<T> a) { return TE<double>{(double)a.m, a.m == T(0) ? 0 : a.e}; }
 template <class T>
 MBX_HD FE fe_from_te(TE<T> a) { return a.m == T(0) ? fe_make(0.0, 0) : fe_make((double)a.m, (int64_t)a.e); }
 
@@ -677,13 +683,20 @@ struct JVal { // J = (r, i) 2^e, (r, i) below 1
 };
 // J' = 2 z J + 1 with z = X + S w in floatexp: the steps where z lies outside
 // the lane type's range (the exact floatexp steps; rare).
-MBX_RARE JVal lane_j_step_fe(FE Xr, FE Xi, FE S, double wr, double wi, int sje, double jr, double ji) {
-    const FE zr = fe_add(Xr, fe_mul_d(S, wr)), zi = fe_add(Xi, fe_mul_d(S, wi));
-    const FE sj = fe_make(0.5, sje), Jr = fe_mul_d(sj, jr), Ji = fe_mul_d(sj, ji);
-    const FE nr = fe_add(fe_scale2(fe_sub(fe_mul(zr, Jr), fe_mul(zi, Ji)), 1), fe_make(0.5, 1));
-    const FE ni = fe_scale2(fe_add(fe_mul(zr, Ji), fe_mul(zi, Jr)), 1);
-    const int64_t e = d_is_zero(nr.m) ? ni.e : (d_is_zero(ni.m) ? nr.e : (nr.e > ni.e ? nr.e : ni.e));
-    return JVal{fe_to_double(fe_make(nr.m, nr.e - e)), fe_to_double(fe_make(ni.m, ni.e - e)), (int)e};
+template <class E>
+MBX_HD JVal lane_j_step_as(FEt<E> Xr, FEt<E> Xi, FEt<E> S, double wr, double wi, int sje, double jr, double ji) {
+    const FEt<E> zr = fe_add(Xr, fe_mul_d(S, wr)), zi = fe_add(Xi, fe_mul_d(S, wi));
+    const FEt<E> sj = fe_make_as<E>(0.5, sje), Jr = fe_mul_d(sj, jr), Ji = fe_mul_d(sj, ji);
+    const FEt<E> nr = fe_add(fe_scale2(fe_sub(fe_mul(zr, Jr), fe_mul(zi, Ji)), 1), fe_make_as<E>(0.5, 1));
+    const FEt<E> ni = fe_scale2(fe_add(fe_mul(zr, Ji), fe_mul(zi, Jr)), 1);
+    const E e = d_is_zero(nr.m) ? ni.e : (d_is_zero(ni.m) ? nr.e : (nr.e > ni.e ? nr.e : ni.e));
+    return JVal{fe_to_double(fe_make_as<E>(nr.m, nr.e - e)), fe_to_double(fe_make_as<E>(ni.m, ni.e - e)), (int)e};
+}
+MBX_RARE JVal lane_j_step_fe(const FE2* X, TE<double> S, double wr, double wi, int sje, double jr, double ji) {
+    const FE Xr = X ? X->re : fe_make(0.0, 0), Xi = X ? X->im : fe_make(0.0, 0);
+    if (te_mid(S.e) && te_mid(sje) && te_mid(Xr.e) && te_mid(Xi.e))
+        return lane_j_step_as(fe_make_as<int>(Xr.m, (int)Xr.e), fe_make_as<int>(Xi.m, (int)Xi.e), fe_make_as<int>(S.m, S.e), wr, wi, sje, jr, ji);
+    return lane_j_step_as(Xr, Xi, fe_make(S.m, S.e), wr, wi, sje, jr, ji);
 }
 // J' = A J + B through a BLA skip, in pairs of floats for both lane types (the
 // FP32 lane rounds the result to float once; FP64 floatexp, as it was formed
@@ -928,21 +941,30 @@ MBX_HD void lane_rebase_to(Lane<T>& L, T zr, T zi) {
 // the new delta (its scale S, 0 when z is, and w).
 struct RebaseFe {
     bool take;
-    FE S;
+    TE<double> S;
     double wr, wi;
 };
-MBX_RARE RebaseFe lane_rebase_fe(FE S, double wr, double wi, FE Xr, FE Xi, bool force) {
-    const FE Swr = fe_mul_d(S, wr), Swi = fe_mul_d(S, wi);
-    const FE zr = fe_add(Xr, Swr), zi = fe_add(Xi, Swi);
-    const FE zrad = fe_add(fe_mul(zr, zr), fe_mul(zi, zi));
-    const FE dz = fe_add(fe_mul(Swr, Swr), fe_mul(Swi, Swi));
-    RebaseFe v{force || fe_abs_less(zrad, dz), fe_make(0.0, 0), 0.0, 0.0};
+template <class E>
+MBX_HD RebaseFe lane_rebase_as(FEt<E> S, double wr, double wi, FEt<E> Xr, FEt<E> Xi, bool force) {
+    const FEt<E> Swr = fe_mul_d(S, wr), Swi = fe_mul_d(S, wi);
+    const FEt<E> zr = fe_add(Xr, Swr), zi = fe_add(Xi, Swi);
+    const FEt<E> zrad = fe_add(fe_mul(zr, zr), fe_mul(zi, zi));
+    const FEt<E> dz = fe_add(fe_mul(Swr, Swr), fe_mul(Swi, Swi));
+    RebaseFe v{force || fe_abs_less(zrad, dz), TE<double>{0.0, 0}, 0.0, 0.0};
     if (!v.take) return v;
-    v.S = fe_sqrt(zrad);
-    if (v.S.m == 0.0) return v;
-    v.wr = fe_to_double(fe_div(zr, v.S));
-    v.wi = fe_to_double(fe_div(zi, v.S));
+    const FEt<E> n = fe_sqrt(zrad);
+    if (n.m == 0.0) return v;
+    v.S = TE<double>{n.m, (int)n.e};
+    v.wr = fe_to_double(fe_div(zr, n));
+    v.wi = fe_to_double(fe_div(zi, n));
     return v;
+}
+// X: the orbit entry, null for 0.
+MBX_RARE RebaseFe lane_rebase_fe(TE<double> S, double wr, double wi, const FE2* X, bool force) {
+    const FE Xr = X ? X->re : fe_make(0.0, 0), Xi = X ? X->im : fe_make(0.0, 0);
+    if (te_mid(S.e) && te_mid(Xr.e) && te_mid(Xi.e))
+        return lane_rebase_as(fe_make_as<int>(S.m, S.e), wr, wi, fe_make_as<int>(Xr.m, (int)Xr.e), fe_make_as<int>(Xi.m, (int)Xi.e), force);
+    return lane_rebase_as(fe_make(S.m, S.e), wr, wi, Xr, Xi, force);
 }
 
 // Common iterations of the FP32 lane without interior detection. The
@@ -1437,8 +1459,7 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
             if (!tiny) {
                 lane_j_advance(L);
             } else { // z outside the lane type's range: in floatexp
-                const FE zero = fe_make(0.0, 0);
-                const JVal v = lane_j_step_fe(L.m ? Zfe[L.rm].re : zero, L.m ? Zfe[L.rm].im : zero, fe_from_te(L.S), (double)L.wr, (double)L.wi, L.SJ.e, (double)L.jr, (double)L.ji);
+                const JVal v = lane_j_step_fe(L.m ? Zfe + L.rm : nullptr, te_double(L.S), (double)L.wr, (double)L.wi, L.SJ.e, (double)L.jr, (double)L.ji);
                 lane_j_set(L, (T)v.r, (T)v.i, v.e);
             }
         }
@@ -1671,13 +1692,12 @@ MBX_HDF int lane_run(Lane<T>& L, int budget, const DeviceFrame& f, const MixedPa
             }
         } else if (decide == 2) {
             ++n_ferebase;
-            const FE zero = fe_make(0.0, 0);
-            const RebaseFe v = lane_rebase_fe(fe_from_te(L.S), (double)L.wr, (double)L.wi, L.m ? Zfe[L.rm].re : zero, L.m ? Zfe[L.rm].im : zero, !per && L.m >= reflen);
+            const RebaseFe v = lane_rebase_fe(te_double(L.S), (double)L.wr, (double)L.wi, L.m ? Zfe + L.rm : nullptr, !per && L.m >= reflen);
             if (v.take) {
                 if (v.S.m == 0.0) {
                     L.wr = L.wi = T(0);
                 } else {
-                    L.S = te_from_fe<T>(v.S);
+                    L.S = te_from_fe<T>(fe_make(v.S.m, v.S.e));
                     L.wr = (T)v.wr;
                     L.wi = (T)v.wi;
                     lane_refresh(L);
