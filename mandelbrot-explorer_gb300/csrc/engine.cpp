@@ -1761,14 +1761,13 @@ int Engine::run_pass(std::vector<uint64_t>* keys, const PixelSet& grid, int mx_r
         p.interior_eps2 = interior_eps2_;
         // A small pass ends with the warp whose samples take longest together.
         // Slow neighbours (chaotic samples beside a minibrot) in one warp, each
-        // on its own path, take up to their sum: up to four warps an SM quarter a
-        // warp takes its samples from four places. 1e-51 view of the tests (6 to 29
-        // % of it interior), 48x104 / 160x120 / 240x180 / 320x240: 104, 107, 126,
-        // 134 ms instead of 124, 146, 170, 170 with 32 neighbours (103, 114, 142,
-        // 145 with lanes that fetched one by one); exteriors at 1e-9 to 1e-30
-        // within 9 % either way. At 400x300, six warps a quarter, 155 instead of
-        // 181 there, but the exteriors 3 to 14 % slower: neighbours from there on.
-        p.spread_tickets = nsm_ * 16;
+        // on its own path, take up to their sum: up to four warps an SM quarter, in
+        // frames with interior, a warp takes its samples from four places. 1e-51
+        // view of the tests (6 to 29 % of it interior), 48x104 / 160x120 / 240x180
+        // / 320x240: 104, 107, 126, 134 ms instead of 124, 146, 170, 170 with 32
+        // neighbours (103, 114, 142, 145 with lanes that fetched one by one). Frames
+        // without interior keep neighbours (four places: 9 % faster to 9 % slower).
+        p.spread_tickets = use_interior_ ? nsm_ * 16 : 0;
         int blocks = std::min((n + threads - 1) / threads, nsm_ * 8);
         e = launch_fp64_pass(f, p, blocks, threads, st_);
     }

@@ -61,3 +61,23 @@ def test_double_path_frames(w, h, cm, sub):
     it, _, en, _ = oracle.render(*args, sub=sub, coloring_method=cm, bailout=c["bailout"])
     assert np.array_equal(r.escape_iteration, en) and np.array_equal(r.iterations < -1.5, it < -1.5)
     np.testing.assert_allclose(r.iterations, it, rtol=1e-6, atol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h,cm,sub", [(5, 3, 0, 1), (48, 104, 0, 1), (304, 256, 0, 1), (311, 251, 64, 1), (60, 33, 1, 3)])
+def test_frames_with_interior(w, h, cm, sub):
+    """Frames whose probe finds interior take the order in the main pass: the cusp
+    of the period-3 minibrot on the needle."""
+    import oracle
+
+    args = ("-1.7499996", "0.0000001", "2000000", w, h, 20000)
+    be = mbx.create_compute_backend("cuda")
+    try:
+        r = mbx.ComputeRequest(*args, sub=sub, coloring_method=cm, bailout=256.0)
+        assert be.compute_status(r) == mbx.OK, be.last_error()
+        assert be.last_stats.as_dict()["used_floatexp"] == 0
+    finally:
+        be.close()
+    it, _, en, _ = oracle.render(*args, sub=sub, coloring_method=cm, bailout=256.0)
+    assert (en < 0).any() and np.array_equal(r.escape_iteration, en) and np.array_equal(r.iterations < -1.5, it < -1.5)
+    np.testing.assert_allclose(r.iterations, it, rtol=1e-6, atol=0)
